@@ -1228,8 +1228,15 @@ struct Context {
             // W[nts-1], writes the other state set and partial sums; its image accumulation is
             // discarded: the pass zeroes the image first)
             tbImg.ensure((size_t)nb * g.isz * 8);
-            const int maxEntR = tb_lists(pl, nb, shots, 2, false);
-            tb_desc(pl, nb, false, true, false, tbW.p, false);
+            // (the traces it injects: the wave's data, or the WEMVA data of a call without any)
+            std::vector<const float*> din(nb);
+            bool inject = true;
+            for (int s = 0; s < nb; s++) {
+                din[s] = dataPtr[s] ? dataPtr[s] : wdataPtr[s];
+                inject &= din[s] != nullptr;
+            }
+            const int maxEntR = tb_lists(pl, nb, shots, inject ? 2 : 0, false);
+            tb_desc(pl, nb, false, inject, false, tbW.p, false, 0, nullptr, 0, din.data());
             a = tb_args(pl, maxEntR, nullptr);
             a.its = g.nts - 2;
             ms = timeMin([&] { tb_launch<TB_ADJ>(pl, nb, a, 0); });
