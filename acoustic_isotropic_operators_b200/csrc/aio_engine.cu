@@ -21,7 +21,7 @@
 
 #include "aio_b200.h"
 #include "aio_kernels.cuh"
-#include "aio_tile.cuh"
+#include "aio_slide.cuh"
 
 namespace aio {
 
@@ -171,6 +171,8 @@ struct Context {
     int smCount = 148;  // streaming multiprocessors of `dev`
     cudaStream_t st = nullptr;
     DevMem v2, rs, taper;
+    float* v2p() const { return v2.as<float>() + (long long)KM_GUARD * g.ip; }  // zero columns around v^2
+    std::vector<float> hv2;  // host copy of v^2 dtw^2, padded grid
     // per-wave buffers
     DevMem pbuf, ringb, ssb, wf1, wf2, wf3, img, lists, desc, sig, dat, aux, model, ext, outv;
     std::vector<ShotDesc> hdesc;
@@ -215,7 +217,7 @@ struct Context {
         AIO_CK(cudaSetDevice(dev));
         AIO_CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
         AIO_CK(cudaDeviceGetAttribute(&smCount, cudaDevAttrMultiProcessorCount, dev));
-        v2.ensure(g.isz * 4);
+        v2.ensure((g.isz + 2LL * KM_GUARD * g.ip) * 4);
         rs.ensure(g.isz * 4);
         taper.ensure(PAD_MAX * 4);
         AIO_CK(cudaMemcpyAsync(taper.p, k.taper, PAD_MAX * 4, cudaMemcpyHostToDevice, st));
@@ -250,9 +252,12 @@ struct Context {
 
     void set_velocity(const float* vel2Dtw2, const float* reflScale) {
         AIO_CK(cudaSetDevice(dev));
-        AIO_CK(cudaMemsetAsync(v2.p, 0, g.isz * 4, st));
+        AIO_CK(cudaMemsetAsync(v2.p, 0, v2.bytes, st));
         AIO_CK(cudaMemsetAsync(rs.p, 0, g.isz * 4, st));
-        if (vel2Dtw2) to_interior(v2.as<float>(), vel2Dtw2, 1, AIO_MEM_HOST);
+        if (vel2Dtw2) {
+            to_interior(v2p(), vel2Dtw2, 1, AIO_MEM_HOST);
+            hv2.assign(vel2Dtw2, vel2Dtw2 + (size_t)g.nz * g.nx);
+        }
         if (reflScale) to_interior(rs.as<float>(), reflScale, 1, AIO_MEM_HOST);
         AIO_CK(cudaStreamSynchronize(st));
     }
@@ -306,7 +311,9 @@ struct Context {
             body();
             return;
         }
-        key.insert(key.end(), {P.freeSurface, P.wavefieldPrecision, P.extension, P.sloth, P.stepper, pdl_mode()});
+        key.insert(key.end(), {P.freeSurface, P.wavefieldPrecision, P.extension, P.sloth, P.stepper, pdl_mode(),
+                               (long long)tbState.p, (long long)tbPart.p, (long long)tbWstage.p, (long long)passW,
+                               (long long)passOut});
         auto it = graphs.find(key);
         if (it != graphs.end()) {
             AIO_CK(cudaGraphLaunch(it->second.exec, st));
@@ -511,7 +518,7 @@ struct Context {
         std::memset(&a, 0, sizeof(a));
         a.g = g;
         a.c = k.c;
-        a.v2 = v2.as<float>();
+        a.v2 = v2p();
         a.taper = taper.as<float>();
         a.shots = desc.as<ShotDesc>();
         a.injTB = -1;
@@ -827,13 +834,13 @@ struct Context {
     // ss[slot] = v2 * (ss[slot] + sum_s m_s(x-s) F_t(x-2s))  (imagingOffsetFwdGpu + scaleSecondarySourceFd)
     void img_offset_fwd(int nb, long long slot, const float* m, const float* F, int t) {
         k_img_offset_fwd<<<ew_grid(nb, g.isz), 256, 0, st>>>(ss_ptr(slot), pairSt(), m, 0, F + (long long)t * g.isz,
-                                                              wfSt(), v2.as<float>(), g.isz, g.ip, g.nxi, g.hExt);
+                                                              wfSt(), v2p(), g.isz, g.ip, g.nxi, g.hExt);
         kcheck();
     }
     // ss[slot] += sum_s m_s(x+s) R_t(x+2s) v2(x+2s)  (imagingOffsetTomoAdjGpu)
     void img_offset_tomo_adj(int nb, long long slot, const float* m, const float* R, int t) {
         k_img_offset_tomo_adj<<<ew_grid(nb, g.isz), 256, 0, st>>>(ss_ptr(slot), pairSt(), m, 0,
-                                                                   R + (long long)t * g.isz, wfSt(), v2.as<float>(),
+                                                                   R + (long long)t * g.isz, wfSt(), v2p(),
                                                                    nullptr, g.isz, g.ip, g.nxi, g.hExt);
         kcheck();
     }
@@ -855,17 +862,17 @@ struct Context {
         const long long mSt = (long long)g.nExt * g.isz, RSt = (long long)OFF_K * g.isz;
         if (P.imageFp64)
             k_img_offset_block<double><<<ew_grid(nb, g.isz), 256, 0, st>>>(
-                img.as<double>(), mSt, offBuf.as<float>(), RSt, F, wfSt(), v2.as<float>(), (int)g.isz, g.ip, g.nxi,
+                img.as<double>(), mSt, offBuf.as<float>(), RSt, F, wfSt(), v2p(), (int)g.isz, g.ip, g.nxi,
                 g.hExt, g.nExt, tlo, thi, wemvaForm ? 1 : 0);
         else
             k_img_offset_block<float><<<ew_grid(nb, g.isz), 256, 0, st>>>(
-                img.as<float>(), mSt, offBuf.as<float>(), RSt, F, wfSt(), v2.as<float>(), (int)g.isz, g.ip, g.nxi,
+                img.as<float>(), mSt, offBuf.as<float>(), RSt, F, wfSt(), v2p(), (int)g.isz, g.ip, g.nxi,
                 g.hExt, g.nExt, tlo, thi, wemvaForm ? 1 : 0);
         kcheck();
     }
 
     void scale_shared(float* m, int nSlices, int mode) {
-        k_scale<<<ew_grid(1, (long long)nSlices * g.isz), 256, 0, st>>>(m, 0, nSlices, v2.as<float>(), rs.as<float>(),
+        k_scale<<<ew_grid(1, (long long)nSlices * g.isz), 256, 0, st>>>(m, 0, nSlices, v2p(), rs.as<float>(),
                                                                          g.isz, mode);
         kcheck();
     }
@@ -875,12 +882,12 @@ struct Context {
     void reduce_images(int nb, int nSlices, int mode, float* out, bool add) {
         const long long n = (long long)nSlices * g.isz;
         if (P.imageFp64) {
-            k_scale_d<<<ew_grid(nb, n), 256, 0, st>>>(img.as<double>(), n, nSlices, v2.as<float>(), rs.as<float>(),
+            k_scale_d<<<ew_grid(nb, n), 256, 0, st>>>(img.as<double>(), n, nSlices, v2p(), rs.as<float>(),
                                                       g.isz, mode);
             kcheck();
             k_sum_shots<double><<<ew_grid(1, n), 256, 0, st>>>(out, img.as<double>(), n, nb, n, add ? 1 : 0);
         } else {
-            k_scale<<<ew_grid(nb, n), 256, 0, st>>>(img.as<float>(), n, nSlices, v2.as<float>(), rs.as<float>(), g.isz,
+            k_scale<<<ew_grid(nb, n), 256, 0, st>>>(img.as<float>(), n, nSlices, v2p(), rs.as<float>(), g.isz,
                                                     mode);
             kcheck();
             k_sum_shots<float><<<ew_grid(1, n), 256, 0, st>>>(out, img.as<float>(), n, nb, n, add ? 1 : 0);
@@ -950,78 +957,197 @@ struct Context {
         drop_graphs();
         for (DevMem* m : call_buffers()) m->release();
     }
-    // k_tile plan: strips of HZ (multiple of 4) output rows, NQ = HZ/4 + 10 row quads,
-    // 8 column pairs per quad, x-chunks of LX columns marched in blocks of 16.
+    // Stepper kernels: marching (k_march), a tile per CTA (k_block), sliding blocks (k_slide, dense-source
+    // modes at sub = 4). A plan: strips of HZ (multiple of 4) output rows, NQ row quads with their halo,
+    // x-chunks of LX columns.
+    enum TBKind { TB_MARCH = 0, TB_TILE = 1, TB_SLIDE = 2 };
     struct TBPlan {
-        int T = KT_T, HZ = 0, nStrips = 0, LX = 0, nChunks = 0, iters = 0, threads = 0, NQ = 0;
+        int T = KT_T, HZ = 0, nStrips = 0, LX = 0, nChunks = 0, NQ = 0;
+        int kind = TB_MARCH;  // stepper kernel
     };
 
     bool tb_enabled() const { return P.stepper != AIO_STEPPER_FINE && g.sub == KT_T; }
+    // The nonlinear and Born passes run blocked whenever a launch's four fine steps span at most two
+    // coarse intervals. (Below that, sub = 2 and 3, a launch would finish two samples.)
+    bool tb_steps() const { return P.stepper != AIO_STEPPER_FINE && g.sub >= KT_T; }
+    bool tb_any_sub() const { return g.sub != KT_T; }
+    int tb_launches() const { return ((g.nts - 1) * g.sub + KT_T - 1) / KT_T; }
+    int tb_parts() const { return tb_any_sub() ? 4 : 2; }  // partial-sum slices per shot
     int wbytes() const { return P.wavefieldPrecision == AIO_WFLD_FP32 ? 4 : 2; }
     bool f16() const { return P.wavefieldPrecision == AIO_WFLD_FP16; }
 
-    // nb: shots of the wave (one CTA column per shot)
-    // Plan of a wave of nb shots: the autotuned plan when one was measured, else the model's.
-    // Plans are tuned per wave size and kernel class: light modes (SRC, NL, ADJR: at most 6
-    // staging slots, no secondary-source rings), heavy modes (SCAT, SCATX, SCATW, ADJX), whose
-    // larger shared-memory footprint changes how many CTAs an SM holds, and the Born receiver
-    // pass (ADJ: 12 staging slots, FP64 image read-modify-write, receivers injected).
-    // The nonlinear forward (NL: sources in, receivers recorded, no stored wavefield) is tuned as
-    // its own class: its single-shot calls are the small, latency-bound waves.
-    enum TBClass { TB_LIGHT = 0, TB_HEAVY = 1, TB_RECV = 2, TB_NLC = 3 };
-    TBPlan tb_plan(int nb, bool heavy = false) const { return tb_plan_c(nb, heavy ? TB_HEAVY : TB_LIGHT); }
+    // Plans are tuned per wave size and kernel class, when a pass of the class first runs: light modes
+    // (SRC, ADJR), heavy modes (SCAT, SCATX: a secondary-source ring in shared memory), those of them that
+    // also store coarse samples (SCATW, ADJX), the Born receiver pass (ADJ)
+    // and the nonlinear forward and adjoint (NL, NLA: no stored wavefield).
+    enum TBClass { TB_LIGHT = 0, TB_HEAVY = 1, TB_RECV = 2, TB_NLC = 3, TB_NLAC = 4, TB_DENSE = 5 };
+    TBPlan tb_plan(int nb) const { return tb_plan_c(nb, TB_LIGHT); }
     TBPlan tb_plan_c(int nb, int cls) const {
-        auto it = tbTuned.find(4 * nb + cls);
+        auto it = tbTuned.find(8 * nb + cls);
         if (it != tbTuned.end()) return it->second;
-        return tb_model_plan(nb, 4 * (KT_MAXQ - 10), P.chunkColumns > 0 ? P.chunkColumns : 0);
+        // forced chunk width: strips of at most 128 rows
+        if (P.chunkColumns > 0)
+            return tb_make_plan((g.nzi + 127) / 128, std::max(1, (g.nxi + P.chunkColumns / 2) / P.chunkColumns));
+        return tb_candidates(nb, cls, TBEntries{}, 1).front();
     }
 
-    // Strips of at most maxHZ rows; x-chunks of about chunkColumns columns, or (0) the chunk
-    // count minimising the modelled time: whole CTA waves over the SMs (one resident CTA per
-    // SM) times the iterations of one CTA (each chunk recomputes 10T warm-up columns), at
-    // least 4 waves preferred so that CTAs of uneven cost (strips holding sources or
-    // receivers) balance out.
-    // minWaves: smallest number of CTA waves (of one CTA per SM) the chunk count is chosen from
-    TBPlan tb_model_plan(int nb, int maxHZ, int chunkColumns, int forceChunks = 0, int minWaves = 4) const {
+    TBPlan tb_make_plan(int nStrips, int nChunks, int kind = TB_MARCH) const {
         TBPlan pl;
-        pl.nStrips = (g.nzi + maxHZ - 1) / maxHZ;
-        pl.HZ = round_up((g.nzi + pl.nStrips - 1) / pl.nStrips, 4);
-        pl.NQ = pl.HZ / 4 + 10;
-        pl.threads = round_up(8 * pl.NQ, 32);
-        if (forceChunks > 0) {
-            pl.nChunks = std::min(forceChunks, g.nxi);
-        } else if (chunkColumns > 0) {
-            pl.nChunks = std::max(1, (g.nxi + chunkColumns / 2) / chunkColumns);
-        } else {
-            double best = 1e300, bestAny = 1e300;
-            int ncAny = 1;
-            pl.nChunks = 0;
-            for (int nc = 1; nc <= std::max(1, g.nxi / 48); nc++) {
-                const int lx = (g.nxi + nc - 1) / nc;
-                const long long ctas = (long long)pl.nStrips * nc * nb;
-                const double cost = (double)((ctas + smCount - 1) / smCount) * ((lx + 10 * pl.T + KT_BX - 1) / KT_BX);
-                if (cost < bestAny * 0.999) {
-                    bestAny = cost;
-                    ncAny = nc;
-                }
-                if (ctas >= (long long)minWaves * smCount && cost < best * 0.999) {
-                    best = cost;
-                    pl.nChunks = nc;
-                }
-            }
-            if (pl.nChunks == 0) pl.nChunks = ncAny;
-        }
-        pl.LX = (g.nxi + pl.nChunks - 1) / pl.nChunks;
-        pl.iters = (pl.LX + 10 * pl.T + KT_BX - 1) / KT_BX;
+        pl.kind = kind;
+        pl.HZ = round_up((g.nzi + nStrips - 1) / nStrips, 4);
+        pl.nStrips = (g.nzi + pl.HZ - 1) / pl.HZ;
+        int rows = 0;
+        for (int s = 0; s < pl.nStrips; s++) rows = std::max(rows, strip_end(pl, s) - strip_begin(pl, s));
+        pl.NQ = (rows + 3) / 4;
+        pl.LX = (g.nxi + nChunks - 1) / nChunks;
+        pl.nChunks = (g.nxi + pl.LX - 1) / pl.LX;
         return pl;
     }
+    // first row of strip s's CTAs (k_march's zb) and the end of the rows they compute
+    int strip_begin(const TBPlan& pl, int s) const { return std::max(pl.kind != TB_MARCH ? -5 * KT_T : 0, s * pl.HZ - 5 * KT_T); }
+    int strip_end(const TBPlan& pl, int s) const {
+        return pl.kind != TB_MARCH ? (s + 1) * pl.HZ + 5 * KT_T : std::min(g.nzi, (s + 1) * pl.HZ + 5 * KT_T);
+    }
 
-    // Measured autotuning of the blocked stepper's plan for waves of nb shots (chunkColumns
-    // == 0): strip heights {128, 112, 96, 80, 64} rows x chunk counts around the model's choices
-    // (at least 4 waves of CTAs, and the cheapest count for any number of waves) are each timed
-    // on the source-pass launch of interval 0 (idempotent: it reads one state set and
-    // overwrites the other, the stored slice 0 and the partial sums), the fastest is cached
-    // for the context. The state is zeroed again afterwards.
+    // Shared-memory and occupancy of plan pl in class cls's largest mode.
+    struct TBEntries {  // largest sparse-entry counts of one CTA: injection slots and recordings
+        int srcIn = 0, recIn = 0, recOut = 0, srcOut = 0, recWarps = 0;
+    };
+    size_t tb_smem(const TBPlan& pl, int cls, const TBEntries& e) const {
+        if (pl.kind == TB_SLIDE) return ks_smem_bytes(pl.NQ, pl.LX, cls == TB_HEAVY ? e.recOut : 0, P.freeSurface);
+        if (pl.kind == TB_TILE)
+            return kb_smem_bytes(cls == TB_HEAVY || cls == TB_DENSE ? TB_SCAT : TB_SRC, pl.NQ, pl.LX,
+                                 cls == TB_NLC                        ? e.srcIn
+                                 : cls == TB_HEAVY || cls == TB_DENSE ? 0
+                                                                      : std::max(e.srcIn, e.recIn));
+        switch (cls) {
+            case TB_NLAC: return km_smem_bytes(TB_NLA, pl.NQ, pl.LX, e.recIn, e.srcOut, std::min(e.srcOut, km_warps(pl.NQ)));
+            case TB_LIGHT: return km_smem_bytes(TB_SRC, pl.NQ, pl.LX, std::max(e.srcIn, e.recIn), 0, 0);
+            case TB_HEAVY: return km_smem_bytes(tb_any_sub() ? TB_SCATG : TB_SCAT, pl.NQ, pl.LX, 0, e.recOut, e.recWarps);
+            case TB_DENSE: return km_smem_bytes(TB_SCATW, pl.NQ, pl.LX, 0, 0, 0);
+            case TB_RECV: return km_smem_bytes(TB_ADJ, pl.NQ, pl.LX, e.recIn, 0, 0);
+            default: return km_smem_bytes(TB_NL, pl.NQ, pl.LX, e.srcIn, e.recOut, e.recWarps);
+        }
+    }
+    static int tb_threads(const TBPlan& pl) {
+        return pl.kind == TB_TILE ? kb_threads(pl.NQ, pl.LX) : (pl.kind == TB_SLIDE ? ks_threads(pl.NQ) : km_threads(pl.NQ));
+    }
+    int tb_occupancy(const TBPlan& pl, int cls, size_t smem) const {
+        if (pl.kind == TB_MARCH && km_threads(pl.NQ) > KM_MAXT) return 0;
+        if (pl.kind == TB_SLIDE && (pl.NQ > KS_MAXQ || (cls != TB_HEAVY && cls != TB_DENSE) || tb_any_sub())) return 0;
+        const void* f = pl.kind == TB_SLIDE  ? (P.freeSurface || pl.NQ > KS_MAXQ_S
+                                                    ? (const void*)k_slide<TB_SCATW, TBW_F32, KS_MAXQ, false>
+                                                    : (const void*)k_slide<TB_SCATW, TBW_F32, KS_MAXQ_S, false>)
+                        : pl.kind == TB_TILE ? (cls == TB_HEAVY || cls == TB_DENSE ? (const void*)k_block<TB_SCATW, TBW_F32, false>
+                                                                                  : (const void*)k_block<TB_ADJ, TBW_F32, false>)
+                        : cls == TB_LIGHT   ? (const void*)k_march<TB_SRC, TBW_F32, false>
+                        : cls == TB_HEAVY ? (const void*)k_march<TB_SCATX, TBW_F32, false>
+                        : cls == TB_DENSE ? (const void*)k_march<TB_SCATW, TBW_F32, false>
+                        : cls == TB_RECV  ? (const void*)k_march<TB_ADJ, TBW_F32, false>
+                        : cls == TB_NLAC  ? (const void*)k_march<TB_NLA, TBW_F32, false>
+                                          : (const void*)k_march<TB_NL, TBW_F32, false>;
+        int smemMax = 0, n = 0;
+        if (cudaDeviceGetAttribute(&smemMax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
+        if (smem > (size_t)smemMax) return 0;
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smemMax);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, tb_threads(pl), smem) != cudaSuccess) return 0;
+        return n;
+    }
+
+    // The `most` plans of the smallest modelled time, cheapest first: whole rounds of the CTAs that an
+    // SM holds; a round lasts one CTA's own latency (about 170 cycles per column and KM_FILL columns of
+    // filling) or the SM's throughput (about 120 cycles per column and warp of a level, filling costing 20
+    // columns), whichever is longer.
+    std::vector<TBPlan> tb_candidates(int nb, int cls, const TBEntries& e, int most) const {
+        std::vector<std::pair<double, TBPlan>> all, some;
+        auto cheaper = [](const std::pair<double, TBPlan>& x, const std::pair<double, TBPlan>& y) { return x.first < y.first; };
+        for (int ns = 1; ns <= std::max(1, g.nzi / 24); ns++) {
+            const TBPlan one = tb_make_plan(ns, 1);
+            if (one.nStrips != ns || km_threads(one.NQ) > KM_MAXT) continue;
+            int lastLX = -1;
+            some.clear();
+            for (int nc = 1; nc <= std::max(1, g.nxi / 4); nc++) {
+                const TBPlan pl = tb_make_plan(ns, nc);
+                if (pl.LX == lastLX) continue;  // the same chunks
+                lastLX = pl.LX;
+                const int occ = tb_occupancy(pl, cls, tb_smem(pl, cls, e));
+                if (occ < 1) continue;
+                const long long perSM = ((long long)pl.nStrips * pl.nChunks * nb + smCount - 1) / smCount;
+                auto round = [&](double k) {
+                    return 2500.0 + std::max((pl.LX + KM_FILL) * 170.0, (pl.LX + 20) * 120.0 * k * km_warps(pl.NQ));
+                };
+                const double t = (double)(perSM / occ) * round(occ) + (perSM % occ ? round((double)(perSM % occ)) : 0.0);
+                some.push_back({t, pl});
+            }
+            std::sort(some.begin(), some.end(), cheaper);  // at most 5 of one strip height
+            all.insert(all.end(), some.begin(), some.begin() + std::min<size_t>(some.size(), 5));
+        }
+        require(!all.empty(), "blocked stepper: no plan fits in shared memory (too many devices per tile)");
+        std::sort(all.begin(), all.end(), cheaper);
+        std::vector<TBPlan> out;
+        for (const auto& c : all) {
+            if ((int)out.size() >= most) break;
+            out.push_back(c.second);
+        }
+        return out;
+    }
+
+    // The `most` k_block plans of the smallest modelled time: rounds of CTAs, each the sum over the levels of
+    // the rounds of its threads (about 600 cycles) after a fixed 3000. Waves that give every SM several
+    // marching CTAs are left to k_march.
+    std::vector<TBPlan> tb_tile_candidates(int nb, int cls, int most) const {
+        std::vector<std::pair<double, TBPlan>> all;
+        std::vector<TBPlan> out;
+        if ((double)nb * g.nzi * g.nxi > 12000.0 * smCount) return out;
+        for (int ns = 1; ns <= std::max(1, g.nzi / 8); ns++) {
+            if (tb_make_plan(ns, 1, TB_TILE).nStrips != ns) continue;
+            int lastLX = -1;
+            for (int nc = 1; nc <= std::max(1, g.nxi / 8); nc++) {
+                const TBPlan pl = tb_make_plan(ns, nc, TB_TILE);
+                if (pl.LX == lastLX || pl.LX % KB_C) continue;
+                lastLX = pl.LX;
+                const size_t smem = tb_smem(pl, cls, TBEntries{});
+                if (smem > 222 * 1024) continue;
+                double t = 3000.0;
+                for (int l = 1; l <= KT_T; l++) {
+                    const int items = (pl.NQ - 2 * (5 * l / 4)) * ((pl.LX + 40 - 10 * l + KB_C - 1) / KB_C), thr = tb_threads(pl);
+                    t += 600.0 * ((items + thr - 1) / thr);
+                }
+                const int occ = std::max(1, std::min((int)(225 * 1024 / (smem + 2048)), 512 / tb_threads(pl)));
+                const long long perSM = ((long long)pl.nStrips * pl.nChunks * nb + smCount - 1) / smCount;
+                // (CTAs sharing an SM hide each other's fixed part)
+                all.push_back({(t - 3000.0) * perSM + 3000.0 * ((perSM + occ - 1) / occ), pl});
+            }
+        }
+        std::sort(all.begin(), all.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
+        for (const auto& c : all)
+            if ((int)out.size() < most) out.push_back(c.second);
+        return out;
+    }
+
+    // k_slide plans of the dense-source classes: per strip height the two chunk counts of the smallest modelled
+    // time, whole rounds of CTAs (one per SM) times the 16-column iterations of one.
+    std::vector<TBPlan> tb_slide_candidates(int nb, int cls) const {
+        std::vector<TBPlan> out;
+        if ((cls != TB_HEAVY && cls != TB_DENSE) || tb_any_sub()) return out;
+        for (int rows : {128, 112, 96, 80, 64, 48}) {
+            const int ns = (g.nzi + rows - 1) / rows;
+            std::vector<std::pair<double, TBPlan>> some;
+            for (int nc = 1; nc <= std::max(1, g.nxi / 16); nc++) {
+                const TBPlan pl = tb_make_plan(ns, nc, TB_SLIDE);
+                const long long ctas = (long long)pl.nStrips * pl.nChunks * nb;
+                some.push_back({(double)((ctas + smCount - 1) / smCount) * ks_iters(pl.LX), pl});
+            }
+            std::stable_sort(some.begin(), some.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
+            for (size_t i = 0; i < some.size() && i < 2; i++) {
+                bool dup = false;
+                for (const TBPlan& o : out) dup |= o.HZ == some[i].second.HZ && o.LX == some[i].second.LX;
+                if (!dup) out.push_back(some[i].second);
+            }
+        }
+        return out;
+    }
+
     std::map<int, TBPlan> tbTuned;
     TBPlan tbLast;  // plan of the most recent blocked launch
 
@@ -1038,134 +1164,99 @@ struct Context {
         return mu;
     }
     std::vector<int> shared_plan_key(int k) const {
-        return {dev, g.nzi, g.nxi, k, P.freeSurface, P.wavefieldPrecision};
+        return {dev, g.nzi, g.nxi, k, P.freeSurface, P.wavefieldPrecision, tb_any_sub() ? 1 : 0};
     }
-    // The shared plans of waves of nb shots, when every class has one that fits these shots.
-    bool tb_take_shared(int nb, const aio_shot* shots, bool nonlinear) {
-        const std::vector<int> classes = nonlinear ? std::vector<int>{TB_NLC} : std::vector<int>{TB_LIGHT, TB_HEAVY, TB_RECV};
-        std::vector<TBPlan> got;
+    // The shared plan of waves of nb shots of a class, when there is one that fits these shots.
+    bool tb_take_shared(int nb, int cls, const aio_shot* shots) {
+        TBPlan pl;
         {
             std::lock_guard<std::mutex> lk(shared_plans_mu());
-            for (int c : classes) {
-                auto it = shared_plans().find(shared_plan_key(4 * nb + c));
-                if (it == shared_plans().end()) return false;
-                got.push_back(it->second);
-            }
+            auto it = shared_plans().find(shared_plan_key(8 * nb + cls));
+            if (it == shared_plans().end()) return false;
+            pl = it->second;
         }
-        for (const TBPlan& pl : got)
-            if (!tb_plan_fits(pl, tb_max_entries(pl, nb, shots))) return false;
-        for (size_t i = 0; i < classes.size(); i++) tbTuned[4 * nb + classes[i]] = got[i];
+        if (tb_occupancy(pl, cls, tb_smem(pl, cls, tb_max_entries(pl, nb, shots))) < 1) return false;
+        tbTuned[8 * nb + cls] = pl;
         return true;
     }
 
-    // Largest sparse-entry counts one CTA of plan pl holds, per kind of pass: sources injected
-    // over the halo region plus receivers recorded in the output region (SRC, NL), receivers
-    // recorded (SCAT, SCATX), receivers injected over the halo region plus sources recorded
-    // (ADJ, ADJR).
-    struct TBEntries {
-        int fwd = 1, scat = 1, adj = 1;
-    };
+    // CTAs (strip range, chunk range) whose region, widened by h points, holds interior point (z, x)
+    template <class F>
+    void tb_for_ctas(const TBPlan& pl, int z, int x, int h, F&& f) const {
+        const int s0 = std::max(0, (z - h) / pl.HZ - 1), s1 = std::min(pl.nStrips - 1, (z + h) / pl.HZ + 1);
+        const int c0 = std::max(0, (x - h) / pl.LX - 1), c1 = std::min(pl.nChunks - 1, (x + h) / pl.LX + 1);
+        for (int s = s0; s <= s1; s++) {
+            if (z < s * pl.HZ - h || z >= std::min((s + 1) * pl.HZ, g.nzi) + h) continue;
+            for (int c = c0; c <= c1; c++)
+                if (x >= c * pl.LX - h && x < std::min((c + 1) * pl.LX, g.nxi) + h) f(s, c);
+        }
+    }
+    static constexpr int TB_INJ = 5 * (KT_T - 1);  // level 1 is needed 15 points around the output region
+
+    // Largest device counts of one CTA (an upper bound of its merged injection slots).
     TBEntries tb_max_entries(const TBPlan& pl, int nb, const aio_shot* shots) const {
-        const int h = 5 * (pl.T - 1);
         const size_t nCTA = (size_t)pl.nStrips * pl.nChunks;
-        std::vector<int> srcHalo(nCTA), srcOut(nCTA), recHalo(nCTA), recOut(nCTA);
+        std::vector<int> n(nCTA);
         TBEntries m;
+        auto most = [&](const int* pos, int cnt, int h, int& out) {
+            std::fill(n.begin(), n.end(), 0);
+            for (int k2 = 0; k2 < cnt; k2++)
+                tb_for_ctas(pl, pos[k2] % g.nz - FAT, pos[k2] / g.nz - FAT, h,
+                            [&](int s, int c) { out = std::max(out, ++n[(size_t)s * pl.nChunks + c]); });
+        };
         for (int s = 0; s < nb; s++) {
-            for (auto* v : {&srcHalo, &srcOut, &recHalo, &recOut}) std::fill(v->begin(), v->end(), 0);
-            auto add = [&](const int* pos, int n, std::vector<int>& halo, std::vector<int>& out) {
-                for (int k2 = 0; k2 < n; k2++) {
-                    const int iz = (int)(pos[k2] % g.nz) - FAT, ix = (int)(pos[k2] / g.nz) - FAT;
-                    for (int st2 = std::max(0, (iz - h) / pl.HZ - 1); st2 <= std::min(pl.nStrips - 1, (iz + h) / pl.HZ + 1); st2++) {
-                        const int z0 = st2 * pl.HZ, z1 = std::min(z0 + pl.HZ, g.nzi);
-                        if (iz < z0 - h || iz >= z1 + h) continue;
-                        for (int ch = std::max(0, (ix - h) / pl.LX - 1); ch <= std::min(pl.nChunks - 1, (ix + h) / pl.LX + 1); ch++) {
-                            const int x0 = ch * pl.LX, x1 = std::min(x0 + pl.LX, g.nxi);
-                            if (ix < x0 - h || ix >= x1 + h) continue;
-                            const size_t c = (size_t)st2 * pl.nChunks + ch;
-                            halo[c]++;
-                            if (ix >= x0 && ix < x1 && iz >= z0 && iz < z1) out[c]++;
-                        }
-                    }
-                }
-            };
-            add(shots[s].sourcesPositionReg, shots[s].nSourcesReg, srcHalo, srcOut);
-            add(shots[s].receiversPositionReg, shots[s].nReceiversReg, recHalo, recOut);
-            for (size_t c = 0; c < nCTA; c++) {
-                m.fwd = std::max(m.fwd, srcHalo[c] + recOut[c]);
-                m.scat = std::max(m.scat, recOut[c]);
-                m.adj = std::max(m.adj, recHalo[c] + srcOut[c]);
+            most(shots[s].sourcesPositionReg, shots[s].nSourcesReg, TB_INJ, m.srcIn);
+            most(shots[s].receiversPositionReg, shots[s].nReceiversReg, TB_INJ, m.recIn);
+            most(shots[s].receiversPositionReg, shots[s].nReceiversReg, 0, m.recOut);
+            most(shots[s].sourcesPositionReg, shots[s].nSourcesReg, 0, m.srcOut);
+            // warps of level 4 (32 row quads each) that record in some CTA: of the widest strip
+            std::vector<unsigned char> has((size_t)pl.nStrips * km_warps(pl.NQ), 0);
+            for (int k2 = 0; k2 < shots[s].nReceiversReg; k2++) {
+                const int z = shots[s].receiversPositionReg[k2] % g.nz - FAT, st2 = z / pl.HZ;
+                if (z >= 0 && z < g.nzi) has[(size_t)st2 * km_warps(pl.NQ) + (z - strip_begin(pl, st2)) / 128] = 1;
             }
+            for (int st2 = 0; st2 < pl.nStrips; st2++)
+                m.recWarps = std::max(m.recWarps, (int)std::count(has.begin() + (size_t)st2 * km_warps(pl.NQ),
+                                                                  has.begin() + (size_t)(st2 + 1) * km_warps(pl.NQ), 1));
         }
         return m;
     }
-    // row quads of the k_tile variant a strip of NQ row quads runs on (the free surface: the
-    // large-strip variant only)
-    int tb_variant(int NQ) const {
-        if (P.freeSurface) return KT_MAXQ;
-        return NQ <= KT_MAXQ_S ? KT_MAXQ_S : (NQ <= KT_MAXQ_M ? KT_MAXQ_M : KT_MAXQ);
-    }
-    // plan pl fits in shared memory in every mode
-    bool tb_plan_fits(const TBPlan& pl, const TBEntries& e) const {
-        int smemMax = 0;
-        if (cudaDeviceGetAttribute(&smemMax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return false;
-        const int mq = tb_variant(pl.NQ);
-        const std::pair<int, int> need[] = {{TB_SRC, e.fwd}, {TB_SCAT, e.scat}, {TB_ADJ, e.adj}, {TB_SCATW, 1}};
-        for (const auto& mn : need)
-            if (kt_smem_bytes(mn.first, pl.threads, pl.iters, mn.second, kt_rs(mq), kt_v2s(mq)) > (size_t)smemMax)
-                return false;
-        return true;
-    }
 
-    // Candidates: strip heights {128 .. 64} rows (and, for waves too small to fill the GPU with
-    // 128-row strips, 48 and 32 rows) x chunk counts around the model's choices; for those small
-    // waves also the chunk counts that give one or two CTAs per SM, with chunks down to 16
-    // columns. nonlinear: the NL class alone is timed (its launch with recording off).
-    void tb_autotune(int nb, const aio_shot* shots, bool nonlinear = false) {
-        if (P.chunkColumns != 0 || tbTuned.count(4 * nb + (nonlinear ? TB_NLC : TB_LIGHT))) return;
-        if (tb_take_shared(nb, shots, nonlinear)) return;
-        const bool small = (long long)tb_model_plan(nb, 128, 0, 0, 1).nStrips * std::max(1, g.nxi / 48) * nb <
-                           2LL * smCount;
-        std::vector<int> heights = {128, 112, 96, 80, 64};
-        if (small) heights.insert(heights.end(), {48, 32});
-        const int maxChunks = std::max(1, g.nxi / (small ? 16 : 32));
+    // Measured autotuning of a class's plan for waves of nb shots (chunkColumns == 0): the dozen
+    // candidates of the smallest modelled time are timed on an idempotent launch of interval 0
+    // (the last interval for ADJ): it reads one state set and overwrites the other, the stored slice
+    // 0 and the partial sums; the fastest is kept for the context and shared with the process.
+    void tb_tune(int nb, const aio_shot* shots, int cls) {
+        if (P.chunkColumns != 0 || tbTuned.count(8 * nb + cls)) return;
+        if (tb_take_shared(nb, cls, shots)) return;
+        // device counts enter the candidates' shared memory: those of a mid-sized tile, then checked
+        // exactly per candidate
         std::vector<TBPlan> cand;
-        for (int maxHZ : heights)
-            for (int minWaves : {4, 1, 0}) {
-                TBPlan m;
-                if (minWaves > 0) {
-                    m = tb_model_plan(nb, maxHZ, 0, 0, minWaves);
-                } else {  // small waves: about one and two CTAs per SM
-                    if (!small) continue;
-                    m = tb_model_plan(nb, maxHZ, 0, 1);
-                    m.nChunks = std::max(1, (int)(smCount / std::max(1LL, (long long)m.nStrips * nb)));
+        for (const TBPlan& pl : tb_tile_candidates(nb, cls, 8))
+            if (tb_occupancy(pl, cls, tb_smem(pl, cls, tb_max_entries(pl, nb, shots))) >= 1) cand.push_back(pl);
+        for (const TBPlan& pl : tb_slide_candidates(nb, cls))
+            if (tb_occupancy(pl, cls, tb_smem(pl, cls, tb_max_entries(pl, nb, shots))) >= 1) cand.push_back(pl);
+        for (const TBPlan& pl : tb_candidates(nb, cls, TBEntries{}, 16))
+            if (tb_occupancy(pl, cls, tb_smem(pl, cls, tb_max_entries(pl, nb, shots))) >= 1) cand.push_back(pl);
+        if (cand.empty()) {  // devices too dense for those: the widest tile that holds its devices
+            for (int ns = 1; ns <= std::max(1, g.nzi / 24) && cand.empty(); ns *= 2)
+                for (int nc = 1; nc <= g.nxi && cand.empty(); nc *= 2) {
+                    const TBPlan pl = tb_make_plan(ns, nc);
+                    if (tb_occupancy(pl, cls, tb_smem(pl, cls, tb_max_entries(pl, nb, shots))) >= 1) cand.push_back(pl);
                 }
-                for (int d : {-2, -1, 0, 1, 2, minWaves == 0 ? m.nChunks : 0}) {
-                    const int nc = m.nChunks + d;
-                    if (nc < 1 || nc > maxChunks) continue;
-                    TBPlan c = tb_model_plan(nb, maxHZ, 0, nc);
-                    bool dup = false;
-                    for (auto& o : cand) dup |= (o.HZ == c.HZ && o.nChunks == c.nChunks);
-                    if (!dup && c.threads <= KT_MAXT && c.NQ <= KT_MAXQ &&
-                        tb_plan_fits(c, tb_max_entries(c, nb, shots)))
-                        cand.push_back(c);
-                }
-            }
-        if (cand.empty()) return;  // the model's plan (tb_plan) then stands
+            require(!cand.empty(), "blocked stepper: too many sparse devices inside one tile");
+        }
         cudaEvent_t e0, e1;
         AIO_CK(cudaEventCreate(&e0));
         AIO_CK(cudaEventCreate(&e1));
-        float bestMs = 1e30f, bestHeavyMs = 1e30f, bestRecvMs = 1e30f;
-        TBPlan best = cand.front(), bestHeavy = cand.front(), bestRecv = cand.front();
         const long long saveLaunches = launches, saveKernels = kernels;
         const int saveProf = profEvery;
         const char* logEnv = std::getenv("AIO_AUTOTUNE_LOG");  // print every candidate's timings
         const bool logTune = logEnv && *logEnv && *logEnv != '0';
         profEvery = 0;
         // Per-launch time: the fastest of three timings of n back-to-back launches (after a timed
-        // warm-up launch: smem carve-out, caches), so that a disturbed timing does not decide the
-        // plan; n makes a timing span >= 0.1 ms (at most 8 launches), which for single-shot
-        // launches of ~20 us keeps event and clock jitter from deciding it while keeping the
-        // tuning of a new wave size short (serving tunes one per grid and wave size).
+        // warm-up launch), so that a disturbed timing does not decide the plan; n makes a timing span
+        // >= 0.1 ms (at most 8 launches).
         auto timeMin = [&](auto launch) {
             AIO_CK(cudaEventRecord(e0, st));
             launch();
@@ -1186,151 +1277,143 @@ struct Context {
             }
             return best2;
         };
+        // the traces a receiver pass injects: the wave's data, or the WEMVA data of a call without any
+        std::vector<const float*> din(nb);
+        bool inject = true;
+        for (int s = 0; s < nb; s++) {
+            din[s] = dataPtr[s] ? dataPtr[s] : wdataPtr[s];
+            inject &= din[s] != nullptr;
+        }
+        // forward recordings are timed too (into the data, which are zeroed again: a class is tuned before the
+        // first pass of a call that records)
+        bool record = cls == TB_HEAVY || cls == TB_NLC;
+        for (int s = 0; s < nb; s++) record &= shots[s].nReceiversReg <= 0 || dataPtr[s] != nullptr;
+        float bestMs = 1e30f;
+        TBPlan best = cand.front();
+        if (cls == TB_RECV) tbImg.ensure((size_t)nb * g.isz * 8);
         for (const TBPlan& pl : cand) {
-            const int maxEnt = tb_lists(pl, nb, shots, 1, false);
+            if (cand.size() == 1) break;
+            const bool src = cls == TB_LIGHT || cls == TB_NLC, recv = (cls == TB_RECV || cls == TB_NLAC) && inject;
+            const TBLists ml = tb_lists(pl, nb, shots, src ? 1 : (recv ? 2 : 0), record ? 1 : 0);
             tb_zero(nb, false);
-            tb_desc(pl, nb, true, false, false, nonlinear ? nullptr : tbW.p, false);
-            KTArgs a = tb_args(pl, maxEnt, nullptr);
-            a.its = 0;
-            if (nonlinear) {  // NL class: the launch without recording (the data stay untouched)
-                const float ms = timeMin([&] { tb_launch<TB_NL>(pl, nb, a, 0); });
-                if (ms < bestMs) {
-                    bestMs = ms;
-                    best = pl;
-                }
-                if (logTune)
-                    std::fprintf(stderr, "aio autotune (NL): shots %d strip %d x %d chunk %d x %d threads %d: %.3f ms\n",
-                                 nb, pl.HZ, pl.nStrips, pl.LX, pl.nChunks, pl.threads, ms);
-                continue;
-            }
-            if (f16()) AIO_CK(cudaMemsetAsync(tbWmax.p, 0, (size_t)nb * g.nts * 4, st));
-            float ms = timeMin([&] { tb_launch<TB_SRC>(pl, nb, a, 0); });
+            // (the heavy class's FP32 sources: whatever the stored wavefield's memory holds, as FP32 slices)
+            const bool dense = cls == TB_HEAVY || cls == TB_DENSE;
+            const int slices = dense ? (wbytes() == 4 ? g.nts : g.nts / 2) : 0;
+            tb_desc(nb, src, recv, record, cls == TB_NLC || cls == TB_NLAC ? nullptr : tbW.p, slices,
+                    cls == TB_DENSE ? tbR.as<float>() : nullptr, TB_RING, din.data());
+            KMArgs a = tb_args(pl, ml, nullptr);
+            if (f16() && cls == TB_LIGHT) AIO_CK(cudaMemsetAsync(tbWmax.p, 0, (size_t)nb * g.nts * 4, st));
+            tb_step(a, 0, cls == TB_RECV || cls == TB_NLAC);
+            a.rSlot = 0;
+            a.rSlot0 = slices > 1 ? 1 : 0;
+            const float ms = timeMin([&] {
+                const bool any = tb_any_sub();
+                if (cls == TB_LIGHT && any) tb_launch_t<TB_SRCG, TBW_F32>(pl, nb, a, 0);
+                else if (cls == TB_LIGHT) tb_launch<TB_SRC>(pl, nb, a, 0);
+                else if (cls == TB_HEAVY && any) tb_launch_t<TB_SCATG, TBW_F32>(pl, nb, a, 0);
+                else if (cls == TB_HEAVY) tb_launch<TB_SCATX>(pl, nb, a, 0);
+                else if (cls == TB_DENSE) tb_launch<TB_SCATW>(pl, nb, a, 0);
+                else if (cls == TB_RECV && any) tb_launch_t<TB_ADJG, TBW_F32>(pl, nb, a, 0);
+                else if (cls == TB_RECV) tb_launch<TB_ADJ>(pl, nb, a, 0);
+                else if (cls == TB_NLAC) tb_launch<TB_NLA>(pl, nb, a, 0);
+                else tb_launch<TB_NL>(pl, nb, a, 0);
+            });
             if (ms < bestMs) {
                 bestMs = ms;
                 best = pl;
             }
-            const float lightMs = ms;
-            // heavy class: the time-lag scattered pass (reads W slices 0, 1 as its sources;
-            // writes only the other state set)
-            const int maxEntH = tb_lists(pl, nb, shots, 0, false);  // before tb_desc: it may move the lists
-            tb_desc(pl, nb, false, false, false, tbW.p, false);
-            a = tb_args(pl, maxEntH, nullptr);
-            a.its = 0;
-            a.rSlot = 0;
-            a.rSlot0 = 1;
-            ms = timeMin([&] { tb_launch<TB_SCATX>(pl, nb, a, 0); });
-            if (ms < bestHeavyMs) {
-                bestHeavyMs = ms;
-                bestHeavy = pl;
-            }
-            const float heavyMs = ms;
-            // receiver class: the Born receiver pass at the last interval (reads state set 0 and
-            // W[nts-1], writes the other state set and partial sums; its image accumulation is
-            // discarded: the pass zeroes the image first)
-            tbImg.ensure((size_t)nb * g.isz * 8);
-            // (the traces it injects: the wave's data, or the WEMVA data of a call without any)
-            std::vector<const float*> din(nb);
-            bool inject = true;
-            for (int s = 0; s < nb; s++) {
-                din[s] = dataPtr[s] ? dataPtr[s] : wdataPtr[s];
-                inject &= din[s] != nullptr;
-            }
-            const int maxEntR = tb_lists(pl, nb, shots, inject ? 2 : 0, false);
-            tb_desc(pl, nb, false, inject, false, tbW.p, false, 0, nullptr, 0, din.data());
-            a = tb_args(pl, maxEntR, nullptr);
-            a.its = g.nts - 2;
-            ms = timeMin([&] { tb_launch<TB_ADJ>(pl, nb, a, 0); });
-            if (ms < bestRecvMs) {
-                bestRecvMs = ms;
-                bestRecv = pl;
-            }
             if (logTune)
-                std::fprintf(stderr,
-                             "aio autotune: shots %d strip %d x %d chunk %d x %d threads %d: light %.3f ms heavy %.3f ms "
-                             "receiver %.3f ms\n",
-                             nb, pl.HZ, pl.nStrips, pl.LX, pl.nChunks, pl.threads, lightMs, heavyMs, ms);
+                std::fprintf(stderr, "aio autotune: class %d shots %d strips %d x %d rows chunks %d x %d columns%s: %.4f ms\n",
+                             cls, nb, pl.nStrips, pl.HZ, pl.nChunks, pl.LX, pl.kind == TB_TILE ? " (tile)" : (pl.kind == TB_SLIDE ? " (slide)" : ""), ms);
         }
+        for (int s = 0; record && s < nb; s++)
+            if (shots[s].nReceiversReg > 0)
+                AIO_CK(cudaMemsetAsync(dataPtr[s], 0, (size_t)shots[s].nReceiversReg * g.nts * 4, st));
         AIO_CK(cudaEventDestroy(e0));
         AIO_CK(cudaEventDestroy(e1));
         launches = saveLaunches;
         kernels = saveKernels;
         profEvery = saveProf;
-        if (nonlinear) {
-            tbTuned[4 * nb + TB_NLC] = best;
-        } else {
-            tbTuned[4 * nb + TB_LIGHT] = best;
-            tbTuned[4 * nb + TB_HEAVY] = bestHeavy;
-            tbTuned[4 * nb + TB_RECV] = bestRecv;
-        }
+        tbTuned[8 * nb + cls] = best;
         std::lock_guard<std::mutex> lk(shared_plans_mu());
-        for (int c : nonlinear ? std::vector<int>{TB_NLC} : std::vector<int>{TB_LIGHT, TB_HEAVY, TB_RECV})
-            shared_plans()[shared_plan_key(4 * nb + c)] = tbTuned[4 * nb + c];
+        shared_plans()[shared_plan_key(8 * nb + cls)] = best;
     }
-
     // Per-CTA sparse lists of every shot of a wave. inj: 0 none, 1 sources, 2 receivers
-    // (over the CTA's recomputed halo region); rec: record receivers (output region).
-    int tb_lists(const TBPlan& pl, int nb, const aio_shot* shots, int inj, bool rec) {
-        std::vector<TBEnt> ents;
-        std::vector<int4> starts((size_t)nb * pl.nStrips * pl.nChunks);
-        const int h = 5 * (pl.T - 1);
-        int maxEnt = 1;
+    // (over the CTA's recomputed halo region); rec: 0 none, 1 receivers, 2 sources recorded (output region). Entries are
+    // sorted by (row quad, column), those recorded by (warp of level 4, column); injected devices of one quad
+    // and column share a slot.
+    struct TBLists {
+        int maxInj = 0, maxRec = 0, recWarps = 0;
+    };
+    TBLists tb_lists(const TBPlan& pl, int nb, const aio_shot* shots, int inj, int rec) {
+        std::vector<KMEnt> ents;
+        const size_t nCTA = (size_t)pl.nStrips * pl.nChunks;
+        passCTAs = (int)nCTA;
+        std::vector<int4> starts((size_t)nb * nCTA);
+        std::vector<std::vector<KMEnt>> cInj(nCTA), cRec(nCTA);
+        TBLists m;
         for (int s = 0; s < nb; s++) {
-            std::vector<std::pair<int, int>> ipos, rpos;  // (interior x, interior z) per device
-            auto collect = [&](const int* pos, int n, std::vector<std::pair<int, int>>& out, const char* what) {
-                out.resize(n);
+            for (auto& v : cInj) v.clear();
+            for (auto& v : cRec) v.clear();
+            auto collect = [&](const int* pos, int n, int h, std::vector<std::vector<KMEnt>>& out, const char* what) {
                 for (int k2 = 0; k2 < n; k2++) {
                     const long long p = pos[k2];
                     const int iz = (int)(p % g.nz), ix = (int)(p / g.nz);
                     require(p >= 0 && ix < g.nx && iz >= FAT && iz < g.nz - FAT && ix >= FAT && ix < g.nx - FAT,
                             std::string(what) + " position " + std::to_string(p) + " is outside the interior grid");
-                    out[k2] = {ix - FAT, iz - FAT};
+                    tb_for_ctas(pl, iz - FAT, ix - FAT, h, [&](int st2, int ch) {
+                        if (pl.kind == TB_SLIDE) {  // k_slide: by column, then row
+                            out[(size_t)st2 * pl.nChunks + ch].push_back(KMEnt{ix - FAT, iz - FAT, k2});
+                            return;
+                        }
+                        const int zrel = iz - FAT - strip_begin(pl, st2), xrel = ix - FAT - (ch * pl.LX - 5 * KT_T);
+                        const int q = zrel / 4;
+                        out[(size_t)st2 * pl.nChunks + ch].push_back(h > 0 ? KMEnt{q << 16 | xrel, zrel & 3, k2}
+                                                                           : KMEnt{(q / 32) << 16 | xrel, (q % 32) << 2 | (zrel & 3), k2});
+                    });
                 }
             };
-            if (inj == 1) collect(shots[s].sourcesPositionReg, shots[s].nSourcesReg, ipos, "source");
-            if (inj == 2) collect(shots[s].receiversPositionReg, shots[s].nReceiversReg, ipos, "receiver");
-            if (rec) collect(shots[s].receiversPositionReg, shots[s].nReceiversReg, rpos, "receiver");
-            for (int st2 = 0; st2 < pl.nStrips; st2++)
-                for (int ch = 0; ch < pl.nChunks; ch++) {
-                    const int z0 = st2 * pl.HZ, z1 = std::min(z0 + pl.HZ, g.nzi);
-                    const int x0 = ch * pl.LX, x1 = std::min(x0 + pl.LX, g.nxi);
-                    std::vector<TBEnt> a1, a2;
-                    for (size_t d = 0; d < ipos.size(); d++) {
-                        const int x = ipos[d].first, z = ipos[d].second;
-                        if (x >= x0 - h && x < x1 + h && z >= z0 - h && z < z1 + h) a1.push_back(TBEnt{x, z, (int)d, 0});
-                    }
-                    for (size_t d = 0; d < rpos.size(); d++) {
-                        const int x = rpos[d].first, z = rpos[d].second;
-                        if (x >= x0 && x < x1 && z >= z0 && z < z1) a2.push_back(TBEnt{x, z, (int)d, 0});
-                    }
-                    auto byCol = [](const TBEnt& A, const TBEnt& B) { return A.col < B.col || (A.col == B.col && A.row < B.row); };
-                    std::sort(a1.begin(), a1.end(), byCol);
-                    std::sort(a2.begin(), a2.end(), byCol);
-                    int4 se;
-                    se.x = (int)ents.size();
-                    ents.insert(ents.end(), a1.begin(), a1.end());
-                    se.y = (int)ents.size();
-                    se.z = se.y;
-                    ents.insert(ents.end(), a2.begin(), a2.end());
-                    se.w = (int)ents.size();
-                    starts[((size_t)s * pl.nStrips + st2) * pl.nChunks + ch] = se;
-                    maxEnt = std::max(maxEnt, se.w - se.x);
+            if (inj == 1) collect(shots[s].sourcesPositionReg, shots[s].nSourcesReg, TB_INJ, cInj, "source");
+            if (inj == 2) collect(shots[s].receiversPositionReg, shots[s].nReceiversReg, TB_INJ, cInj, "receiver");
+            if (rec == 1) collect(shots[s].receiversPositionReg, shots[s].nReceiversReg, 0, cRec, "receiver");
+            if (rec == 2) collect(shots[s].sourcesPositionReg, shots[s].nSourcesReg, 0, cRec, "source");
+            for (size_t c = 0; c < nCTA; c++) {
+                auto byKey = [](const KMEnt& A, const KMEnt& B) { return A.key < B.key || (A.key == B.key && A.slot < B.slot); };
+                std::sort(cInj[c].begin(), cInj[c].end(), byKey);
+                std::sort(cRec[c].begin(), cRec[c].end(), byKey);
+                int slots = 0;
+                for (size_t e = 0; e < cInj[c].size(); e++) {
+                    if (e == 0 || cInj[c][e].key != cInj[c][e - 1].key) slots++;
+                    cInj[c][e].slot |= (slots - 1) << 2;
                 }
+                m.maxInj = std::max(m.maxInj, slots);
+                m.maxRec = std::max(m.maxRec, (int)cRec[c].size());
+                int warps = 0;
+                for (size_t e = 0; e < cRec[c].size(); e++) warps += e == 0 || (cRec[c][e].key >> 16) != (cRec[c][e - 1].key >> 16);
+                m.recWarps = std::max(m.recWarps, warps);
+                int4 se;
+                se.x = (int)ents.size();
+                ents.insert(ents.end(), cInj[c].begin(), cInj[c].end());
+                se.y = se.z = (int)ents.size();
+                ents.insert(ents.end(), cRec[c].begin(), cRec[c].end());
+                se.w = (int)ents.size();
+                starts[(size_t)s * nCTA + c] = se;
+            }
         }
-        require(maxEnt <= 4096, "too many sparse devices inside one blocked-stepper tile");
-        tbEnt.ensure(std::max<size_t>(ents.size(), 1) * sizeof(TBEnt));
+        tbEnt.ensure(std::max<size_t>(ents.size(), 1) * sizeof(KMEnt));
         tbStart.ensure(starts.size() * sizeof(int4));
         if (!ents.empty())
-            AIO_CK(cudaMemcpyAsync(tbEnt.p, ents.data(), ents.size() * sizeof(TBEnt), cudaMemcpyHostToDevice, st));
+            AIO_CK(cudaMemcpyAsync(tbEnt.p, ents.data(), ents.size() * sizeof(KMEnt), cudaMemcpyHostToDevice, st));
         AIO_CK(cudaMemcpyAsync(tbStart.p, starts.data(), starts.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
-        return maxEnt;
+        return m;
     }
 
     void tb_alloc(int nb, bool needImg) {
         require(g.isz < (1LL << 31), "interior slice too large for 32-bit in-slice offsets");
         tbState.ensure((size_t)nb * 4 * g.isz * 4);
-        tbPart.ensure((size_t)nb * 2 * g.isz * 4);
+        tbPart.ensure((size_t)nb * tb_parts() * g.isz * 4);
         if (needImg) tbImg.ensure((size_t)nb * g.isz * 8);
-        tbDesc.ensure((size_t)2 * nb * sizeof(TBShot));
+        tbDesc.ensure((size_t)nb * sizeof(TBShot));
         if (f16()) {
             tbWscale.ensure((size_t)nb * g.nts * 4);
             tbWmax.ensure((size_t)nb * g.nts * 4);
@@ -1339,91 +1422,140 @@ struct Context {
         }
     }
 
-    // Descriptor pairs: version v reads state/part set v and writes set 1-v
-    // (partSwap=true: the ADJ part ordering, see tb_adj_pass).
+    // Per-shot descriptors and array bases of a pass (launch version v reads state and partial-sum
+    // set v and writes set 1-v).
     // wSlices: coarse slices per shot in W (the stored wavefield: nts; a secondary-source ring: its length)
-    // out / outSlices: per-shot slices written by ADJR / SCATW / ADJX (default: the LAG_K ring tbR)
+    // out / outSlices: per-shot slices written by ADJR / SCATW / ADJX
     // dataIn: traces injected when injData (default: the wave's data)
     // W: the stored source wavefield (elements of wbytes()) or, with wSlices > 0, an FP32 ring of
     // wSlices secondary-source slices
-    void tb_desc(const TBPlan& pl, int nb, bool injSources, bool injData, bool recData, void* W, bool partFlip,
-                 int wSlices = 0, float* out = nullptr, int outSlices = 0, const float* const* dataIn = nullptr) {
+    void tb_desc(int nb, bool injSources, bool injData, bool recData, void* W, int wSlices = 0, float* out = nullptr,
+                 int outSlices = 0, const float* const* dataIn = nullptr, const std::vector<float*>* srcOut = nullptr) {
         const int wElem = wSlices > 0 ? 4 : wbytes();
         if (wSlices <= 0) wSlices = g.nts;
-        if (!out && tbR.p) {
-            out = tbR.as<float>();
-            outSlices = LAG_K;
-        }
-        std::vector<TBShot> d(2 * (size_t)nb);
-        const int nCTA = pl.nStrips * pl.nChunks;
-        for (int v = 0; v < 2; v++)
-            for (int s = 0; s < nb; s++) {
-                TBShot& t = d[(size_t)v * nb + s];
-                std::memset(&t, 0, sizeof(t));
-                float* base = tbState.as<float>() + (size_t)s * 4 * g.isz;
-                t.cur = base + (size_t)(2 * v) * g.isz;
-                t.old = base + (size_t)(2 * v + 1) * g.isz;
-                t.ncur = base + (size_t)(2 * (1 - v)) * g.isz;
-                t.nold = base + (size_t)(2 * (1 - v) + 1) * g.isz;
-                float* pb = tbPart.as<float>() + (size_t)s * 2 * g.isz;
-                const int vin = partFlip ? (v ^ 1) : v;
-                t.part = pb + (size_t)vin * g.isz;
-                t.partOut = pb + (size_t)(1 - vin) * g.isz;
-                t.injSig = injSources ? srcSig[s] : (injData ? (dataIn ? dataIn[s] : dataPtr[s]) : nullptr);
-                t.injLd = injSources ? g.ntw : g.nts;
-                t.recSig = recData ? dataPtr[s] : nullptr;
-                t.recLd = g.nts;
-                t.entStart = tbStart.as<int4>() + (size_t)s * nCTA;
-                t.ent = tbEnt.as<TBEnt>();
-                t.W = W ? (void*)((char*)W + (size_t)s * wSlices * g.isz * wElem) : nullptr;
-                t.img = tbImg.p ? tbImg.as<double>() + (size_t)s * g.isz : nullptr;
-                t.imgF = tbImg.p ? tbImg.as<float>() + (size_t)s * g.isz : nullptr;
-                t.rcoarse = out ? out + (size_t)s * outSlices * g.isz : nullptr;
-                if (f16()) {
-                    t.wscale = tbWscale.as<float>() + (size_t)s * g.nts;
-                    t.wmax = tbWmax.as<unsigned>() + (size_t)s * g.nts;
-                    t.wstage = tbWstage.as<float>() + (size_t)s * 2 * g.isz;
-                    t.wover = tbWover.as<unsigned>();
-                }
+        passW = W;
+        passWShot = (long long)wSlices * g.isz;
+        passOut = out;
+        passOutShot = (long long)outSlices * g.isz;
+        std::vector<TBShot> d(nb);
+        for (int s = 0; s < nb; s++) {
+            TBShot& t = d[s];
+            std::memset(&t, 0, sizeof(t));
+            t.injSig = injSources ? srcSig[s] : (injData ? (dataIn ? dataIn[s] : dataPtr[s]) : nullptr);
+            t.injLd = injSources ? g.ntw : g.nts;
+            t.recSig = recData ? dataPtr[s] : nullptr;
+            t.recLd = g.nts;
+            if (srcOut) {  // every fine step at the sources
+                t.recSig = (*srcOut)[s];
+                t.recLd = g.ntw;
             }
+            t.entStart = tbStart.as<int4>() + (size_t)s * passCTAs;
+            t.ent = tbEnt.as<KMEnt>();
+            t.W = W ? (void*)((char*)W + (size_t)s * passWShot * wElem) : nullptr;
+            if (f16()) {
+                t.wscale = tbWscale.as<float>() + (size_t)s * g.nts;
+                t.wmax = tbWmax.as<unsigned>() + (size_t)s * g.nts;
+                t.wstage = tbWstage.as<float>() + (size_t)s * 2 * g.isz;
+                t.wover = tbWover.as<unsigned>();
+            }
+        }
         AIO_CK(cudaMemcpyAsync(tbDesc.p, d.data(), d.size() * sizeof(TBShot), cudaMemcpyHostToDevice, st));
     }
+    void* passW = nullptr;  // arrays of the current pass (tb_desc); its CTAs per shot (tb_lists)
+    int passCTAs = 0;
+    float* passOut = nullptr;
+    long long passWShot = 0, passOutShot = 0;
 
-    KTArgs tb_args(const TBPlan& pl, int maxEnt, const float* dm) const {
-        KTArgs a;
+    KMArgs tb_args(const TBPlan& pl, const TBLists& ml, const float* dm) const {
+        KMArgs a;
         std::memset(&a, 0, sizeof(a));
         a.g = g;
         a.c = k.c;
-        a.v2 = v2.as<float>();
+        a.v2 = v2p();
         a.taper = taper.as<float>();
         a.dm = dm;
+        a.shots = tbDesc.as<TBShot>();
         std::copy(k.h, k.h + 2 * (SUB_MAX + 1), a.h);
         a.HZ = pl.HZ;
         a.LX = pl.LX;
         a.nStrips = pl.nStrips;
         a.nChunks = pl.nChunks;
         a.NQ = pl.NQ;
-        a.iters = pl.iters;
-        a.maxEnt = maxEnt;
+        a.maxInj = ml.maxInj;
+        a.maxRec = ml.maxRec;
+        a.recWarps = ml.recWarps;
         a.wStride = g.isz;
         a.imgF32 = P.imageFp64 ? 0 : 1;
+        a.W = passW;
+        a.wShot = passWShot;
+        a.out = passOut;
+        a.outShot = passOutShot;
+        a.img = tbImg.p;
+        a.wstage = tbWstage.as<float>();
+        a.partShot = (long long)tb_parts() * g.isz;
         return a;
     }
+    // Launch L of a pass: fine steps f0 = 4L .. f0 + 3 and the weights of their levels in the coarse samples
+    // (h, F/src/nonlinearShotsGpuFunctions.cu:155-170) and of the secondary sources in them. Forward fine
+    // step it2 = 1..sub of interval its adds h[it2] to sample its and h[H+it2] to its+1 and takes the
+    // sources of its, its+1 by h[it2-1], h[H+it2-1]; adjoint step it2 = sub-1..0 adds h[it2], h[H+it2] and
+    // takes h[it2+1], h[H+it2+1].
+    void tb_step(KMArgs& a, int L, bool back) const {
+        a.f0 = KT_T * L;
+        a.F = (g.nts - 1) * g.sub;
+        const int iv0 = a.f0 / g.sub;
+        a.its = back ? g.nts - 2 - iv0 : iv0;
+        a.c0 = back ? g.nts - 1 - iv0 : iv0;
+        a.last = a.f0 + KT_T >= a.F ? 1 : 0;
+        a.nfin = (a.last || (a.f0 + KT_T) / g.sub > iv0) ? 1 : 0;
+        a.nK = 2;
+        std::memset(a.w, 0, sizeof(a.w));
+        std::memset(a.hs, 0, sizeof(a.hs));
+        for (int l = 0; l < KT_T && a.f0 + l < a.F; l++) {
+            const int f = a.f0 + l, i = f / g.sub - iv0, r = f % g.sub;
+            const int it2 = back ? g.sub - 1 - r : r + 1;
+            a.w[i][l] = back ? k.h[g.H + it2] : k.h[it2];
+            a.w[i + 1][l] = back ? k.h[it2] : k.h[g.H + it2];
+            a.hs[i][l] = back ? k.h[it2 + 1] : k.h[it2 - 1];
+            a.hs[i + 1][l] = back ? k.h[g.H + it2 + 1] : k.h[g.H + it2 - 1];
+            a.nK = i + 2;
+        }
+    }
 
-    template <int MODE, int WP, int MAXQ, bool FS = false>
-    void tb_launch_q(const TBPlan& pl, int nb, KTArgs& a, int v) {
-        const size_t smem = kt_smem_bytes(MODE, pl.threads, pl.iters, a.maxEnt, kt_rs(MAXQ), kt_v2s(MAXQ));
+    template <int MODE, int WP>
+    void tb_launch_t(const TBPlan& pl, int nb, KMArgs& a, int v) {
+        if (P.freeSurface) tb_launch_f<MODE, WP, true>(pl, nb, a, v);
+        else tb_launch_f<MODE, WP, false>(pl, nb, a, v);
+    }
+    template <int MODE, int WP, bool FS>
+    void tb_launch_f(const TBPlan& pl, int nb, KMArgs& a, int v) {
+        constexpr bool slideMode = tb_scatlike(MODE) && MODE != TB_SCATG;
+        const size_t smem = pl.kind == TB_TILE    ? kb_smem_bytes(MODE, pl.NQ, pl.LX, a.maxInj)
+                            : pl.kind == TB_SLIDE ? ks_smem_bytes(pl.NQ, pl.LX, a.maxRec, FS)
+                                                  : km_smem_bytes(MODE, pl.NQ, pl.LX, a.maxInj, a.maxRec, a.recWarps);
         static int attrDev = -1;
         static int smemMax = 0;
         if (attrDev != dev) {
+            const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
             AIO_CK(cudaDeviceGetAttribute(&smemMax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-            AIO_CK(cudaFuncSetAttribute(k_tile<MODE, WP, MAXQ, FS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smemMax));
+            AIO_CK(cudaFuncSetAttribute(k_march<MODE, WP, FS>, attr, smemMax));
+            AIO_CK(cudaFuncSetAttribute(k_block<MODE, WP, FS>, attr, smemMax));
+            if constexpr (slideMode) {
+                AIO_CK(cudaFuncSetAttribute(k_slide<MODE, WP, KS_MAXQ, FS>, attr, smemMax));
+                if (!FS) AIO_CK(cudaFuncSetAttribute(k_slide<MODE, WP, KS_MAXQ_S, false>, attr, smemMax));
+            }
             attrDev = dev;
         }
         require(smem <= (size_t)smemMax, "blocked stepper: shared memory plan of " + std::to_string(smem) +
                                              " bytes exceeds the device limit (too many devices per tile)");
-        require(pl.NQ <= MAXQ && pl.threads <= (8 * MAXQ + 31) / 32 * 32, "blocked stepper: strip taller than the ring");
-        a.shots = tbDesc.as<TBShot>() + (size_t)v * nb;
+        require(pl.kind == TB_TILE || (pl.kind == TB_SLIDE ? slideMode && pl.NQ <= KS_MAXQ : km_threads(pl.NQ) <= KM_MAXT),
+                "blocked stepper: strip taller than the CTA");
+        a.cur = tbState.as<float>() + (size_t)(2 * v) * g.isz;
+        a.old = a.cur + g.isz;
+        a.ncur = tbState.as<float>() + (size_t)(2 * (1 - v)) * g.isz;
+        a.nold = a.ncur + g.isz;
+        a.part = tbPart.as<float>() + (size_t)v * g.isz;  // (sub > 4: the next sample's sums 2 slices behind)
+        a.partOut = tbPart.as<float>() + (size_t)(1 - v) * g.isz;
         tbLast = pl;
         const bool timed = profEvery > 0 && (launches % profEvery) == 0;
         std::pair<cudaEvent_t, cudaEvent_t> ev{};
@@ -1433,7 +1565,7 @@ struct Context {
         }
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(pl.nStrips, pl.nChunks, nb);
-        cfg.blockDim = dim3(pl.threads);
+        cfg.blockDim = dim3(tb_threads(pl));
         cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
         cudaLaunchAttribute at[1];
@@ -1442,8 +1574,17 @@ struct Context {
         cfg.attrs = at;
         const int pm = pdl_mode();
         cfg.numAttrs = pm ? 1 : 0;
-        a.relIter = pm == 1 ? 0 : pl.iters - 1;
-        AIO_CK(cudaLaunchKernelEx(&cfg, k_tile<MODE, WP, MAXQ, FS>, a));
+        a.relEarly = pm == 1 ? 1 : 0;
+        if (pl.kind == TB_TILE) {
+            AIO_CK(cudaLaunchKernelEx(&cfg, k_block<MODE, WP, FS>, a));
+        } else if (pl.kind == TB_SLIDE) {
+            if constexpr (slideMode) {
+                if (FS || pl.NQ > KS_MAXQ_S) AIO_CK(cudaLaunchKernelEx(&cfg, k_slide<MODE, WP, KS_MAXQ, FS>, a));
+                else AIO_CK(cudaLaunchKernelEx(&cfg, k_slide<MODE, WP, KS_MAXQ_S, false>, a));
+            }
+        } else {
+            AIO_CK(cudaLaunchKernelEx(&cfg, k_march<MODE, WP, FS>, a));
+        }
         if (timed) {
             AIO_CK(cudaEventRecord(ev.second, st));
             evBusy.push_back(ev);
@@ -1452,20 +1593,13 @@ struct Context {
         launches++;
         kernels++;
     }
-    // Short strips (<= 64 rows) and mid strips (<= 80 rows) use the variants with narrower
-    // rings (two CTAs per SM); taller strips the large one.
-    template <int MODE, int WP>
-    void tb_launch_t(const TBPlan& pl, int nb, KTArgs& a, int v) {
-        if (P.freeSurface) tb_launch_q<MODE, WP, KT_MAXQ, true>(pl, nb, a, v);
-        else if (pl.NQ <= KT_MAXQ_S) tb_launch_q<MODE, WP, KT_MAXQ_S>(pl, nb, a, v);
-        else if (pl.NQ <= KT_MAXQ_M) tb_launch_q<MODE, WP, KT_MAXQ_M>(pl, nb, a, v);
-        else tb_launch_q<MODE, WP, KT_MAXQ>(pl, nb, a, v);
-    }
     template <int MODE>
-    void tb_launch(const TBPlan& pl, int nb, KTArgs& a, int v) {
+    void tb_launch(const TBPlan& pl, int nb, KMArgs& a, int v) {
         // the dense-source modes read FP32 rings of secondary sources, and the receiver-sample
         // pass reads no stored wavefield: those run on FP32 whatever the stored precision
-        if (MODE == TB_SCATX || MODE == TB_SCATW || MODE == TB_ADJX || MODE == TB_ADJR) tb_launch_t<MODE, TBW_F32>(pl, nb, a, v);
+        if (MODE == TB_SCATX || MODE == TB_SCATW || MODE == TB_ADJX || MODE == TB_ADJR || MODE == TB_NL ||
+            MODE == TB_NLA)
+            tb_launch_t<MODE, TBW_F32>(pl, nb, a, v);
         else if (P.wavefieldPrecision == AIO_WFLD_BF16) tb_launch_t<MODE, TBW_BF16>(pl, nb, a, v);
         else if (P.wavefieldPrecision == AIO_WFLD_FP16) tb_launch_t<MODE, TBW_F16>(pl, nb, a, v);
         else tb_launch_t<MODE, TBW_F32>(pl, nb, a, v);
@@ -1473,7 +1607,7 @@ struct Context {
 
     void tb_zero(int nb, bool img) {
         AIO_CK(cudaMemsetAsync(tbState.p, 0, (size_t)nb * 4 * g.isz * 4, st));
-        AIO_CK(cudaMemsetAsync(tbPart.p, 0, (size_t)nb * 2 * g.isz * 4, st));
+        AIO_CK(cudaMemsetAsync(tbPart.p, 0, (size_t)nb * tb_parts() * g.isz * 4, st));
         if (img) AIO_CK(cudaMemsetAsync(tbImg.p, 0, (size_t)nb * g.isz * 8, st));
     }
 
@@ -1483,24 +1617,25 @@ struct Context {
     // previous slice's max (kt_f16_spec_scale); if any slice outgrew its scale's headroom the
     // pass is run again with every slice staged in FP32 and quantized with its exact max.
     void tb_src_pass(int nb, const aio_shot* shots, bool nonlinear, bool exactF16 = false) {
-        tb_autotune(nb, shots, nonlinear);
+        tb_tune(nb, shots, nonlinear ? TB_NLC : TB_LIGHT);
         const TBPlan pl = nonlinear ? tb_plan_c(nb, TB_NLC) : tb_plan(nb);
-        const int maxEnt = tb_lists(pl, nb, shots, 1, nonlinear);
+        const TBLists ml = tb_lists(pl, nb, shots, 1, nonlinear);
         tb_zero(nb, false);
-        tb_desc(pl, nb, true, false, nonlinear, nonlinear ? nullptr : tbW.p, false);
-        KTArgs a = tb_args(pl, maxEnt, nullptr);
+        tb_desc(nb, true, false, nonlinear, nonlinear ? nullptr : tbW.p);
+        KMArgs a = tb_args(pl, ml, nullptr);
         const bool spec = !nonlinear && f16() && !exactF16;
         a.f16spec = spec ? 1 : 0;
         if (!nonlinear && f16()) AIO_CK(cudaMemsetAsync(tbWmax.p, 0, (size_t)nb * g.nts * 4, st));
         if (spec) AIO_CK(cudaMemsetAsync(tbWover.p, 0, 4, st));
         tbLast = pl;
-        graph_loop({1, nonlinear, nb, pl.HZ, pl.nStrips, pl.LX, pl.nChunks, maxEnt, (long long)tbDesc.p,
+        graph_loop({1, nonlinear, nb, pl.kind, pl.HZ, pl.nStrips, pl.LX, pl.nChunks, ml.maxInj, ml.maxRec, ml.recWarps, (long long)tbDesc.p,
                     (long long)tbW.p, a.f16spec, P.wavefieldPrecision},
                    [&] {
-                       for (int its = 0; its < g.nts - 1; its++) {
-                           a.its = its;
-                           if (nonlinear) tb_launch<TB_NL>(pl, nb, a, its & 1);
-                           else tb_launch<TB_SRC>(pl, nb, a, its & 1);
+                       for (int L = 0; L < tb_launches(); L++) {
+                           tb_step(a, L, false);
+                           if (nonlinear) tb_launch<TB_NL>(pl, nb, a, L & 1);
+                           else if (tb_any_sub()) tb_launch_t<TB_SRCG, TBW_F32>(pl, nb, a, L & 1);
+                           else tb_launch<TB_SRC>(pl, nb, a, L & 1);
                        }
                    });
         if (!nonlinear && f16()) {  // last two slices and the per-slice scales
@@ -1522,19 +1657,21 @@ struct Context {
     // field the secondary sources dm * W come from (default: the source wavefield tbW).
     // A caller's W (the tomo forward's scattered field) is FP32 whatever the stored precision.
     void tb_scat_pass(int nb, const aio_shot* shots, const float* dm, const float* W = nullptr) {
-        const TBPlan pl = tb_plan(nb, true);
-        const int maxEnt = tb_lists(pl, nb, shots, 0, true);
+        tb_tune(nb, shots, TB_HEAVY);
+        const TBPlan pl = tb_plan_c(nb, TB_HEAVY);
+        const TBLists ml = tb_lists(pl, nb, shots, 0, true);
         tb_zero(nb, false);
-        tb_desc(pl, nb, false, false, true, W ? (void*)W : tbW.p, false, W ? g.nts : 0);
-        KTArgs a = tb_args(pl, maxEnt, dm);
+        tb_desc(nb, false, false, true, W ? (void*)W : tbW.p, W ? g.nts : 0);
+        KMArgs a = tb_args(pl, ml, dm);
         tbLast = pl;
-        graph_loop({2, nb, pl.HZ, pl.nStrips, pl.LX, pl.nChunks, maxEnt, (long long)tbDesc.p, (long long)dm,
+        graph_loop({2, nb, pl.kind, pl.HZ, pl.nStrips, pl.LX, pl.nChunks, ml.maxInj, ml.maxRec, ml.recWarps, (long long)tbDesc.p, (long long)dm,
                     (long long)(W ? (const void*)W : tbW.p), P.wavefieldPrecision},
                    [&] {
-                       for (int its = 0; its < g.nts - 1; its++) {
-                           a.its = its;
-                           if (W) tb_launch_t<TB_SCAT, TBW_F32>(pl, nb, a, its & 1);
-                           else tb_launch<TB_SCAT>(pl, nb, a, its & 1);
+                       for (int L = 0; L < tb_launches(); L++) {
+                           tb_step(a, L, false);
+                           if (tb_any_sub()) tb_launch_t<TB_SCATG, TBW_F32>(pl, nb, a, L & 1);
+                           else if (W) tb_launch_t<TB_SCAT, TBW_F32>(pl, nb, a, L & 1);
+                           else tb_launch<TB_SCAT>(pl, nb, a, L & 1);
                        }
                    });
     }
@@ -1543,20 +1680,50 @@ struct Context {
     // Launch L handles interval its = nts-2-L: it reads the partial R(its+1) written by
     // launch L-1 and writes R(its); state ping-pongs with L.
     void tb_adj_pass(int nb, const aio_shot* shots) {
+        tb_tune(nb, shots, TB_RECV);
         const TBPlan pl = tb_plan_c(nb, TB_RECV);
-        const int maxEnt = tb_lists(pl, nb, shots, 2, false);
+        const TBLists ml = tb_lists(pl, nb, shots, 2, false);
         tb_zero(nb, true);
-        tb_desc(pl, nb, false, true, false, tbW.p, false);
-        KTArgs a = tb_args(pl, maxEnt, nullptr);
+        tb_desc(nb, false, true, false, tbW.p);
+        KMArgs a = tb_args(pl, ml, nullptr);
         tbLast = pl;
-        graph_loop({3, nb, pl.HZ, pl.nStrips, pl.LX, pl.nChunks, maxEnt, (long long)tbDesc.p, (long long)tbW.p,
+        graph_loop({3, (long long)tbImg.p, nb, pl.kind, pl.HZ, pl.nStrips, pl.LX, pl.nChunks, ml.maxInj, ml.maxRec, ml.recWarps, (long long)tbDesc.p, (long long)tbW.p,
                     P.wavefieldPrecision},
                    [&] {
-                       for (int L = 0; L < g.nts - 1; L++) {
-                           a.its = g.nts - 2 - L;
-                           tb_launch<TB_ADJ>(pl, nb, a, L & 1);
+                       for (int L = 0; L < tb_launches(); L++) {
+                           tb_step(a, L, true);
+                           if (tb_any_sub()) tb_launch_t<TB_ADJG, TBW_F32>(pl, nb, a, L & 1);
+                           else tb_launch<TB_ADJ>(pl, nb, a, L & 1);
                        }
                    });
+    }
+
+    // Nonlinear adjoint (F/src/nonlinearShotsGpuFunctions.cu:616-641) on U = v2 * p: every fine step of U / v2
+    // at the sources.
+    void tb_nla_pass(int nb, const aio_shot* shots, const std::vector<float*>& srcOut) {
+        tb_alloc(nb, false);
+        tb_tune(nb, shots, TB_NLAC);
+        const TBPlan pl = tb_plan_c(nb, TB_NLAC);
+        const TBLists ml = tb_lists(pl, nb, shots, 2, 2);
+        tb_zero(nb, false);
+        tb_desc(nb, false, true, false, nullptr, 0, nullptr, 0, nullptr, &srcOut);
+        KMArgs a = tb_args(pl, ml, nullptr);
+        tbLast = pl;
+        graph_loop({4, nb, pl.kind, pl.HZ, pl.nStrips, pl.LX, pl.nChunks, ml.maxInj, ml.maxRec, ml.recWarps, (long long)tbDesc.p}, [&] {
+            for (int L = 0; L < tb_launches(); L++) {
+                tb_step(a, L, true);
+                tb_launch<TB_NLA>(pl, nb, a, L & 1);
+            }
+        });
+    }
+    // v^2 is positive at every source position (U / v2 is the field there)
+    bool sources_move(int nShots, const aio_shot* shots) const {
+        for (int s = 0; s < nShots; s++)
+            for (int k2 = 0; k2 < shots[s].nSourcesReg; k2++) {
+                const long long p = shots[s].sourcesPositionReg[k2];
+                if (p < 0 || p >= (long long)hv2.size() || !(hv2[p] > 0.f)) return false;
+            }
+        return true;
     }
 
     // Receiver pass of the extended (time-lag) adjoint (F/src/BornExtShotsGpuFunctions.cu:1525-1675)
@@ -1567,10 +1734,10 @@ struct Context {
     // with subsurface offsets k_img_offset_block (imagingOffsetAdjGpu, :397-411).
     void tb_adjx_pass(int nb, const aio_shot* shots) {
         const TBPlan pl = tb_plan(nb);
-        const int maxEnt = tb_lists(pl, nb, shots, 2, false);
+        const TBLists ml = tb_lists(pl, nb, shots, 2, false);
         tb_zero(nb, false);
-        tb_desc(pl, nb, false, true, false, tbW.p, false);
-        KTArgs a = tb_args(pl, maxEnt, nullptr);
+        tb_desc(nb, false, true, false, tbW.p, 0, tbR.as<float>(), LAG_K);
+        KMArgs a = tb_args(pl, ml, nullptr);
         const long long mSt = (long long)g.nExt * g.isz;
         const int nP = LAG_NP;
         const size_t lagSmem = (size_t)lag_window_len(g.hExt) * nP * 4;
@@ -1621,7 +1788,7 @@ struct Context {
             kcheck();
         };
         for (int L = 0; L < g.nts - 1; L++) {
-            a.its = g.nts - 2 - L;
+            tb_step(a, L, true);
             const int t = a.its + 1;
             a.rSlot = t % LAG_K;
             a.rSlot0 = 0;
@@ -1637,11 +1804,12 @@ struct Context {
     // read by TB_SCATX at slots its and its+1.
     void tb_scatx_pass(int nb, const aio_shot* shots, const float* ext, const float* F = nullptr) {
         const int ring = 2 * LAG_K;
-        const TBPlan pl = tb_plan(nb, true);
-        const int maxEnt = tb_lists(pl, nb, shots, 0, true);
+        tb_tune(nb, shots, TB_HEAVY);
+        const TBPlan pl = tb_plan_c(nb, TB_HEAVY);
+        const TBLists ml = tb_lists(pl, nb, shots, 0, true);
         tb_zero(nb, false);
-        tb_desc(pl, nb, false, false, true, tbSS.p, false, ring);
-        KTArgs a = tb_args(pl, maxEnt, nullptr);
+        tb_desc(nb, false, false, true, tbSS.p, ring);
+        KMArgs a = tb_args(pl, ml, nullptr);
         const int nP = LAG_NP;
         const size_t lagSmem = (size_t)lag_window_len(g.hExt) * nP * 4;
         static int ssAttr = -1;
@@ -1664,7 +1832,7 @@ struct Context {
                 for (int t = tlo; t <= thi; t++)
                     k_img_offset_fwd<<<ew_grid(nb, g.isz), 256, 0, st>>>(
                         tbSS.as<float>() + (long long)(t % ring) * g.isz, rSt, ext, 0, Fs + (long long)t * g.isz,
-                        wfSt(), v2.as<float>(), g.isz, g.ip, g.nxi, g.hExt);
+                        wfSt(), v2p(), g.isz, g.ip, g.nxi, g.hExt);
                 kcheck();
                 return;
             }
@@ -1690,7 +1858,7 @@ struct Context {
         for (int its = 0; its < g.nts - 1; its++) {
             if (its == 0) sources(0);
             if ((its + 1) % LAG_K == 0) sources(its + 1);  // next block, before ss(its+1) is read
-            a.its = its;
+            tb_step(a, its, false);
             a.rSlot = its % ring;
             a.rSlot0 = (its + 1) % ring;
             tb_launch<TB_SCATX>(pl, nb, a, its & 1);
@@ -1840,17 +2008,18 @@ struct Context {
     // F/src/tomoExtShotsGpuFunctions.cu:1554-1656,2442-2527, F/src/wemvaExtShotsGpuFunctions.cu:961-1037.
     // Lag sources are formed a block of LAG_K steps ahead; sample rings are imaged per block.
     void tb_dense_fwd(int nb, const aio_shot* shots, const TBSrc& src, const TBOut& out) {
-        const TBPlan pl = tb_plan(nb, true);
-        const int maxEnt = tb_lists(pl, nb, shots, 0, false);
+        tb_tune(nb, shots, TB_DENSE);
+        const TBPlan pl = tb_plan_c(nb, TB_DENSE);
+        const TBLists ml = tb_lists(pl, nb, shots, 0, false);
         tb_zero(nb, false);
         const bool lagSrc = src.ext != nullptr;
         // zero-lag sources straight from a 16-bit source field: W is that field (wSlices 0: the
         // stored precision's element size), read with its per-slice scales
         const int wp = lagSrc ? TBW_F32 : src.wp;
-        tb_desc(pl, nb, false, false, false, lagSrc ? tbSS.p : const_cast<void*>(src.F), false,
+        tb_desc(nb, false, false, false, lagSrc ? tbSS.p : const_cast<void*>(src.F),
                 lagSrc ? TB_RING : (wp == TBW_F32 ? g.nts : 0), out.full ? out.full : tbR.as<float>(),
                 out.full ? g.nts : TB_RING);
-        KTArgs a = tb_args(pl, maxEnt, lagSrc ? nullptr : src.dm);
+        KMArgs a = tb_args(pl, ml, lagSrc ? nullptr : src.dm);
         int lo = 0;  // lowest sample not yet imaged
         for (int its = 0; its < g.nts - 1; its++) {
             if (lagSrc) {
@@ -1864,7 +2033,7 @@ struct Context {
             }
             a.oA = out.full ? its : its % TB_RING;
             a.oB = out.full ? its + 1 : (its + 1) % TB_RING;
-            a.its = its;
+            tb_step(a, its, false);
             if (wp == TBW_BF16) tb_launch_t<TB_SCATW, TBW_BF16>(pl, nb, a, its & 1);
             else if (wp == TBW_F16) tb_launch_t<TB_SCATW, TBW_F16>(pl, nb, a, its & 1);
             else tb_launch_t<TB_SCATW, TBW_F32>(pl, nb, a, its & 1);
@@ -1881,14 +2050,15 @@ struct Context {
     // Adjoint-time dense pass (adj_dense_pass on the blocked stepper, TB_ADJX) on U-form sources:
     // F/src/tomoExtShotsGpuFunctions.cu:2619-2700, F/src/wemvaExtShotsGpuFunctions.cu:1038-1121.
     void tb_dense_adj(int nb, const aio_shot* shots, const TBSrc& src, const TBOut& out) {
-        const TBPlan pl = tb_plan(nb, true);
-        const int maxEnt = tb_lists(pl, nb, shots, 0, false);
+        tb_tune(nb, shots, TB_DENSE);
+        const TBPlan pl = tb_plan_c(nb, TB_DENSE);
+        const TBLists ml = tb_lists(pl, nb, shots, 0, false);
         tb_zero(nb, false);
         const bool lagSrc = src.ext != nullptr;
         require(lagSrc || src.wp == TBW_F32, "adjoint dense pass: zero-lag sources come from an FP32 field");
-        tb_desc(pl, nb, false, false, false, lagSrc ? tbSS.p : const_cast<void*>(src.F), false,
+        tb_desc(nb, false, false, false, lagSrc ? tbSS.p : const_cast<void*>(src.F),
                 lagSrc ? TB_RING : g.nts, out.full ? out.full : tbR.as<float>(), out.full ? g.nts : TB_RING);
-        KTArgs a = tb_args(pl, maxEnt, lagSrc ? nullptr : src.dm);
+        KMArgs a = tb_args(pl, ml, lagSrc ? nullptr : src.dm);
         int srcLo = g.nts;   // lowest source sample in the ring
         int hi = g.nts - 1;  // highest sample not yet imaged
         for (int L = 0; L < g.nts - 1; L++) {
@@ -1907,7 +2077,7 @@ struct Context {
             }
             a.oA = 0;
             a.oB = out.full ? its + 1 : (its + 1) % TB_RING;
-            a.its = its;
+            tb_step(a, L, true);
             tb_launch_t<TB_ADJX, TBW_F32>(pl, nb, a, L & 1);
             if (!out.full) {
                 const int t = its + 1;
@@ -1924,12 +2094,12 @@ struct Context {
     // F/src/tomoExtShotsGpuFunctions.cu:1481-1515, on TB_ADJR).
     void tb_rec_full(int nb, const aio_shot* shots, const float* const* data, float* R) {
         const TBPlan pl = tb_plan(nb);
-        const int maxEnt = tb_lists(pl, nb, shots, 2, false);
+        const TBLists ml = tb_lists(pl, nb, shots, 2, false);
         tb_zero(nb, false);
-        tb_desc(pl, nb, false, true, false, nullptr, false, 0, R, g.nts, data);
-        KTArgs a = tb_args(pl, maxEnt, nullptr);
+        tb_desc(nb, false, true, false, nullptr, 0, R, g.nts, data);
+        KMArgs a = tb_args(pl, ml, nullptr);
         for (int L = 0; L < g.nts - 1; L++) {
-            a.its = g.nts - 2 - L;
+            tb_step(a, L, true);
             a.rSlot = a.its + 1;
             a.rSlot0 = 0;
             tb_launch_t<TB_ADJR, TBW_F32>(pl, nb, a, L & 1);
@@ -1951,12 +2121,12 @@ struct Context {
     // slice's exact unit (max / 2^15). The FP32 field of nts slices is never held.
     void tb_src_dt2_16(int nb, const aio_shot* shots) {
         static_assert(TB_RING >= 2 * KT_DT2_B, "the block reads the slice before it and the slice after it");
-        tb_autotune(nb, shots, false);
+        tb_tune(nb, shots, TB_LIGHT);
         const TBPlan pl = tb_plan(nb);
-        const int maxEnt = tb_lists(pl, nb, shots, 1, false);
+        const TBLists ml = tb_lists(pl, nb, shots, 1, false);
         tb_zero(nb, false);
-        tb_desc(pl, nb, true, false, false, tbSS.p, false, TB_RING);
-        KTArgs a = tb_args(pl, maxEnt, nullptr);
+        tb_desc(nb, true, false, false, tbSS.p, TB_RING);
+        KMArgs a = tb_args(pl, ml, nullptr);
         a.wRing = TB_RING;
         const int wp = src_wp();
         if (wp == TBW_F16) AIO_CK(cudaMemsetAsync(tbWmax.p, 0, (size_t)nb * g.nts * 4, st));
@@ -1978,12 +2148,12 @@ struct Context {
             kcheck();
         };
         tbLast = pl;
-        graph_loop({11, nb, pl.HZ, pl.nStrips, pl.LX, pl.nChunks, maxEnt, (long long)tbDesc.p, (long long)tbSS.p,
+        graph_loop({11, nb, pl.kind, pl.HZ, pl.nStrips, pl.LX, pl.nChunks, ml.maxInj, ml.maxRec, ml.recWarps, (long long)tbDesc.p, (long long)tbSS.p,
                     (long long)tbW.p, (long long)tbR.p, wp},
                    [&] {
                        int lo = 0;  // first slice of d2/dt2 not yet formed
                        for (int its = 0; its < g.nts - 1; its++) {
-                           a.its = its;
+                           tb_step(a, its, false);
                            tb_launch_t<TB_SRC, TBW_F32>(pl, nb, a, its & 1);
                            // W[its] is final (and W[nts-1] after the last launch): d2/dt2 of the
                            // slices up to `ready` can be formed
@@ -2122,7 +2292,7 @@ struct Context {
     // wavefield, :310-395 — only a batch of one shot returns it).
     void nonlinear_forward(int nShots, const aio_shot* shots, int mem, float* wavefieldOut) {
         begin_call();
-        if (tb_enabled() && !wavefieldOut) return nonlinear_forward_tb(nShots, shots, mem);
+        if (tb_steps() && !wavefieldOut) return nonlinear_forward_tb(nShots, shots, mem);
         Needs n;
         n.nWavefields = wavefieldOut ? 1 : 0;
         for (int s0 = 0; s0 < nShots;) {
@@ -2139,10 +2309,11 @@ struct Context {
     // Nonlinear adjoint (F/src/nonlinearShotsGpuFunctions.cu:579-652 / :653-737).
     void nonlinear_adjoint(int nShots, const aio_shot* shots, int mem, float* wavefieldOut) {
         begin_call();
+        const bool blocked = tb_steps() && !wavefieldOut && sources_move(nShots, shots);
         Needs n;
         n.nWavefields = wavefieldOut ? 1 : 0;
         for (int s0 = 0; s0 < nShots;) {
-            const int nb = wave_size(n, nShots - s0, shots + s0);
+            const int nb = blocked ? tb_wave_size(nShots - s0, shots + s0, false, false) : wave_size(n, nShots - s0, shots + s0);
             setup_wave(n, nb, shots + s0, mem, true, false);
             std::vector<float*> srcOut(nb);
             std::vector<const float*> din(dataPtr.begin(), dataPtr.end());
@@ -2154,8 +2325,11 @@ struct Context {
                 if (sh.nSourcesReg > 0) AIO_CK(cudaMemsetAsync(o, 0, (size_t)sh.nSourcesReg * g.ntw * 4, st));
                 srcOut[s] = o;
             }
-            adj_sparse_pass(nb, din, &srcOut, wavefieldOut ? ACC_FULL : ACC_NONE, wavefieldOut ? &wf1 : nullptr,
-                            [](int, long long) {});
+            if (blocked)
+                tb_nla_pass(nb, shots + s0, srcOut);
+            else
+                adj_sparse_pass(nb, din, &srcOut, wavefieldOut ? ACC_FULL : ACC_NONE, wavefieldOut ? &wf1 : nullptr,
+                                [](int, long long) {});
             if (mem == AIO_MEM_HOST)
                 for (int s = 0; s < nb; s++) {
                     const aio_shot& sh = shots[s0 + s];
@@ -2187,7 +2361,7 @@ struct Context {
             maxSrc = std::max(maxSrc, shots[s].nSourcesReg);
             maxRec = std::max(maxRec, shots[s].nReceiversReg);
         }
-        long long per = 6LL * g.isz * 4 + (wavefield ? (long long)g.nts * g.isz * wbytes() : 0) +
+        long long per = (4LL + tb_parts()) * g.isz * 4 + (wavefield ? (long long)g.nts * g.isz * wbytes() : 0) +
                         (wavefield && f16() ? 2LL * g.isz * 4 + 8LL * g.nts : 0) +
                         (image ? g.isz * 8LL : 0) + (long long)maxSrc * g.ntw * 4 + 2LL * maxRec * g.nts * 4 +
                         2 * g.hsz * 4 + 2 * g.isz * 4 + (1 << 16);
@@ -2231,10 +2405,10 @@ struct Context {
             // (FP32 images when imageFp64 = 0: accumulated in the receiver pass as the reference does)
             const long long nI = g.isz;
             if (P.imageFp64)
-                k_scale_d<<<ew_grid(nb, nI), 256, 0, st>>>(tbImg.as<double>(), nI, 1, v2.as<float>(), rs.as<float>(),
+                k_scale_d<<<ew_grid(nb, nI), 256, 0, st>>>(tbImg.as<double>(), nI, 1, v2p(), rs.as<float>(),
                                                            g.isz, 3);
             else
-                k_scale<<<ew_grid(nb, nI), 256, 0, st>>>(tbImg.as<float>(), nI, 1, v2.as<float>(), rs.as<float>(),
+                k_scale<<<ew_grid(nb, nI), 256, 0, st>>>(tbImg.as<float>(), nI, 1, v2p(), rs.as<float>(),
                                                          g.isz, 3);
             kcheck();
             auto sum = [&](float* dst, int s, int n, int add) {
@@ -2264,7 +2438,7 @@ struct Context {
     void born_adjoint_shots(float* const* images, int nShots, const aio_shot* shots, int mem) {
         begin_call();
         for (int s = 0; s < nShots; s++) require(images && images[s], "per-shot image output is NULL");
-        if (tb_enabled()) return born_adjoint_tb(nullptr, 0, nShots, shots, mem, images);
+        if (tb_steps()) return born_adjoint_tb(nullptr, 0, nShots, shots, mem, images);
         for (int s = 0; s < nShots; s++) born_adjoint(images[s], 0, 1, shots + s, mem);
     }
 
@@ -2288,7 +2462,7 @@ struct Context {
     // Born forward (F/src/BornShotsGpuFunctions.cu:260-388).
     void born_forward(const float* model, int nShots, const aio_shot* shots, int mem) {
         begin_call();
-        if (tb_enabled()) return born_forward_tb(model, nShots, shots, mem);
+        if (tb_steps()) return born_forward_tb(model, nShots, shots, mem);
         Needs n;
         n.nWavefields = 1;
         n.ss = true;
@@ -2312,7 +2486,7 @@ struct Context {
     // summed on the device.
     void born_adjoint(float* modelOut, int add, int nShots, const aio_shot* shots, int mem) {
         begin_call();
-        if (tb_enabled()) return born_adjoint_tb(modelOut, add, nShots, shots, mem);
+        if (tb_steps()) return born_adjoint_tb(modelOut, add, nShots, shots, mem);
         Needs n;
         n.nWavefields = 1;
         n.nImg = 1;
@@ -2429,7 +2603,7 @@ struct Context {
         std::vector<const float*> din(dataPtr.begin(), dataPtr.end());
         adj_sparse_pass(1, din, nullptr, ACC_RING, nullptr, [&](int t, long long slot) {
             k_record_scale<<<ew_grid(1, g.isz), 256, 0, st>>>(wf2.as<float>() + (long long)t * g.isz, ring_ptr(slot),
-                                                               rs.as<float>(), v2.as<float>(), g.isz);
+                                                               rs.as<float>(), v2p(), g.isz);
             kcheck();
             img_adj(1, slot, W, t);
         });
@@ -2489,7 +2663,7 @@ struct Context {
         std::vector<const float*> din(dataPtr.begin(), dataPtr.end());
         adj_sparse_pass(1, din, nullptr, ACC_RING, nullptr, [&](int t, long long slot) {
             k_record_scale<<<ew_grid(1, g.isz), 256, 0, st>>>(wf2.as<float>() + (long long)t * g.isz, ring_ptr(slot),
-                                                               offsets() ? nullptr : rs.as<float>(), v2.as<float>(),
+                                                               offsets() ? nullptr : rs.as<float>(), v2p(),
                                                                g.isz);
             kcheck();
             if (offsets()) img_offset_adj_block(1, slot, W, t, false, true);
@@ -2556,7 +2730,7 @@ struct Context {
         float* dst = wf3.as<float>() + (long long)t * g.isz;
         if (scaled) {
             AIO_CK(cudaMemsetAsync(dst, 0, (size_t)g.isz * 4, st));
-            k_record_scale<<<ew_grid(1, g.isz), 256, 0, st>>>(dst, ring_ptr(slot), nullptr, v2.as<float>(), g.isz);
+            k_record_scale<<<ew_grid(1, g.isz), 256, 0, st>>>(dst, ring_ptr(slot), nullptr, v2p(), g.isz);
             kcheck();
         } else {
             AIO_CK(cudaMemcpyAsync(dst, ring_ptr(slot), (size_t)g.isz * 4, cudaMemcpyDeviceToDevice, st));

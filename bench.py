@@ -202,7 +202,7 @@ def run_reference(args):
 
 def kernel_name(args, w):
     if args.stepper != "fine" and w.sub == 4:
-        return "k_tile (interval-blocked stepper, one launch per coarse interval)"
+        return "k_march / k_slide (interval steppers, one launch per coarse interval)"
     return "k_step (fused fine-step stepper)"
 
 
@@ -623,7 +623,7 @@ def main():
             traffic = None
 
     try:  # plan of the timed region's last launch (a receiver pass of the last wave)
-        plan = ctx.blocked_plan(0) if kernel_name(args, w).startswith("k_tile") else None
+        plan = ctx.blocked_plan(0) if kernel_name(args, w).startswith("k_march") else None
     except Exception:
         plan = None
 

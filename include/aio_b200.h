@@ -82,7 +82,8 @@ typedef struct {
 #define AIO_EXT_TIME 0      /* time lags (the *TimeShots* drivers) */
 #define AIO_EXT_OFFSET 1    /* horizontal subsurface offsets (the *OffsetShots* drivers; per-fine-step stepper) */
 
-#define AIO_STEPPER_AUTO 0      /* interval-blocked where available (sub == 4), else per fine step */
+#define AIO_STEPPER_AUTO 0      /* four fine steps per launch where available (sub == 4; nonlinear and Born
+                                   operators: sub >= 4), else per fine step */
 #define AIO_STEPPER_FINE 1      /* one fused launch per fine step (the reference's schedule) */
 #define AIO_STEPPER_BLOCKED 2   /* one launch per coarse interval, 2-D register tiles (requires sub == 4) */
 
