@@ -1,0 +1,90 @@
+"""The interval steppers at the edges of their tiles: strips of one row quad and of a remainder, chunks
+narrower than a block, idle lanes, one and many strips, launches that straddle a coarse interval
+(sub > 4), against the per-fine-step stepper. Both are FP32 evaluations of one scheme: relative L2 below
+2e-5 (each is within 1e-5 of the FP64 oracle at these lengths, tests/test_gpu_parity.py)."""
+import numpy as np
+import pytest
+
+from cases import interior_mask, make_case, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+# nzi, nxi, shots: below one warp of row quads, exactly one (128 rows) and one row more, two strips, odd sizes
+SIZES = [(11, 23, 1), (33, 40, 3), (128, 37, 2), (129, 61, 1), (301, 45, 2), (67, 530, 1), (530, 30, 1)]
+
+
+def _pair(nzi, nxi, sub, fs, shots, chunk=0, **kw):
+    import orc
+    from acoustic_isotropic_operators_b200.batch import Context
+    c = make_case(seed=nzi + sub, nzi=nzi, nxi=nxi, nts=14, sub=sub, minPad=6, nshots=shots, vmin=1500.0, vmax=1900.0)
+    s = c.scheme
+    k = orc.constants(s, c.vel, dtype=np.float32)
+    mk = lambda **a: Context(s.nz, s.nx, s.nts, s.dts, s.sub, s.dz, s.dx, s.minPad, k["v2"], k["rs"], free_surface=fs,  # noqa: E731
+                             **kw, **a)
+    return c, mk(chunk_columns=chunk), mk(stepper="fine")
+
+
+def _shots(c, data=None):
+    from acoustic_isotropic_operators_b200.batch import Shot
+    return [Shot(c.src_pos[i], c.rec_pos[i], c.sig[i], None if data is None else data[i]) for i in range(len(c.src_pos))]
+
+
+@pytest.mark.parametrize("fs", [0, 1])
+@pytest.mark.parametrize("sub", [4, 5, 7, 8])
+@pytest.mark.parametrize("nzi,nxi,shots", SIZES)
+def test_against_fine_steps(nzi, nxi, shots, sub, fs):
+    """Timed plans, and (chunk 17) marching strips of at most 128 rows."""
+    for chunk in (0, 17):
+        c, blocked, fine = _pair(nzi, nxi, sub, fs, shots, chunk)
+        data = [c.rng.standard_normal((len(r), c.scheme.nts)).astype(np.float32) for r in c.rec_pos]
+        model = (c.rng.standard_normal((c.nx, c.nz)) * interior_mask(c.nx, c.nz)).astype(np.float32)
+        out = []
+        for ctx in (blocked, fine):
+            out.append([np.concatenate([x.ravel() for x in ctx.nonlinear_forward(_shots(c))]),
+                        np.concatenate([x.ravel() for x in ctx.nonlinear_adjoint(_shots(c, data))]),
+                        np.concatenate([x.ravel() for x in ctx.born_forward(model, _shots(c))]),
+                        ctx.born_adjoint(_shots(c, data)).ravel().copy()])
+            ctx.close()
+        for name, a, b in zip(("nl fwd", "nl adj", "born fwd", "born adj"), *out):
+            assert np.linalg.norm(b) > 0
+            assert rel_l2(a, b) < 2e-5, (name, chunk)
+
+
+@pytest.mark.parametrize("nzi,nxi,shots", SIZES)
+def test_dense_source_passes(nzi, nxi, shots):
+    """Tomo and WEMVA (dense sources, stored samples), timed plans."""
+    c, blocked, fine = _pair(nzi, nxi, 4, 0, shots, nExt=3)
+    ext = (c.rng.standard_normal((3, c.nx, c.nz)) * interior_mask(c.nx, c.nz)).astype(np.float32)
+    data = [c.rng.standard_normal((len(r), c.scheme.nts)).astype(np.float32) for r in c.rec_pos]
+    out = []
+    for ctx in (blocked, fine):
+        out.append([np.concatenate([x.ravel() for x in ctx.tomo_forward(ext[1], ext, _shots(c))]),
+                    ctx.tomo_adjoint(ext, _shots(c, data)).ravel().copy()])
+        ctx.close()
+    for a, b in zip(*out):
+        assert np.linalg.norm(b) > 0
+        assert rel_l2(a, b) < 1e-4  # (second differences of FP32 fields)
+
+
+@pytest.mark.parametrize("sub", [4, 6])
+def test_devices_everywhere(sub):
+    """A receiver on every third grid point and two devices on one point: more entries per CTA than the
+    preferred tiles hold, recordings and injections in every warp."""
+    import orc
+    from acoustic_isotropic_operators_b200.batch import Context, Shot
+    c = make_case(seed=9, nzi=140, nxi=90, nts=10, sub=sub, minPad=6, nshots=1, vmin=1500.0, vmax=1900.0)
+    s = c.scheme
+    k = orc.constants(s, c.vel, dtype=np.float32)
+    pos = np.array([ix * s.nz + iz for ix in range(5, s.nx - 5) for iz in range(5, s.nz - 5)][::3], np.int32)
+    pos = np.concatenate([pos, pos[:1]])
+    data = (c.rng.standard_normal((len(pos), s.nts)) * 1e-2).astype(np.float32)
+    out = []
+    for stepper in ("auto", "fine"):
+        ctx = Context(s.nz, s.nx, s.nts, s.dts, s.sub, s.dz, s.dx, s.minPad, k["v2"], k["rs"], stepper=stepper)
+        out.append([ctx.nonlinear_forward([Shot(c.src_pos[0], pos, c.sig[0])])[0].copy(),
+                    ctx.nonlinear_adjoint([Shot(c.src_pos[0], pos, None, data)])[0].copy(),
+                    ctx.born_adjoint([Shot(c.src_pos[0], pos, c.sig[0], data)]).copy()])
+        ctx.close()
+    np.testing.assert_array_equal(out[0][0][0], out[0][0][-1])
+    for a, b in zip(*out):
+        assert rel_l2(a, b) < 2e-5
