@@ -968,7 +968,7 @@ struct Context {
 
     bool tb_enabled() const { return P.stepper != AIO_STEPPER_FINE && g.sub == KT_T; }
     // The nonlinear and Born passes run blocked whenever a launch's four fine steps span at most two
-    // coarse intervals. (Below that, sub = 2 and 3, a launch would finish two samples.)
+    // coarse intervals. (Below that, sub = 2 and 3, a launch would finish two samples.) See tb_runs.
     bool tb_steps() const { return P.stepper != AIO_STEPPER_FINE && g.sub >= KT_T; }
     bool tb_any_sub() const { return g.sub != KT_T; }
     int tb_launches() const { return ((g.nts - 1) * g.sub + KT_T - 1) / KT_T; }
@@ -1196,10 +1196,16 @@ struct Context {
     // Largest device counts of one CTA (an upper bound of its merged injection slots).
     TBEntries tb_max_entries(const TBPlan& pl, int nb, const aio_shot* shots) const {
         const size_t nCTA = (size_t)pl.nStrips * pl.nChunks;
-        std::vector<int> n(nCTA);
+        std::vector<int> n(nCTA), pts;
         TBEntries m;
         auto most = [&](const int* pos, int cnt, int h, int& out) {
             std::fill(n.begin(), n.end(), 0);
+            if (h > 0) {  // injected devices of one point share a slot
+                pts.assign(pos, pos + cnt);
+                std::sort(pts.begin(), pts.end());
+                cnt = (int)(std::unique(pts.begin(), pts.end()) - pts.begin());
+                pos = pts.data();
+            }
             for (int k2 = 0; k2 < cnt; k2++)
                 tb_for_ctas(pl, pos[k2] % g.nz - FAT, pos[k2] / g.nz - FAT, h,
                             [&](int s, int c) { out = std::max(out, ++n[(size_t)s * pl.nChunks + c]); });
@@ -1222,12 +1228,64 @@ struct Context {
         return m;
     }
 
+    // The devices of these shots fit plan pl's shared memory: by their number alone, or counted per CTA.
+    bool tb_fits(const TBPlan& pl, int nb, int cls, const aio_shot* shots) const {
+        int smemMax = 0;
+        if (cudaDeviceGetAttribute(&smemMax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return false;
+        TBEntries e;
+        for (int s = 0; s < nb; s++) {
+            e.srcIn = e.srcOut = std::max(e.srcIn, shots[s].nSourcesReg);
+            e.recIn = e.recOut = std::max(e.recIn, shots[s].nReceiversReg);
+        }
+        e.recWarps = km_warps(pl.NQ);
+        return tb_smem(pl, cls, e) <= (size_t)smemMax ||
+               tb_smem(pl, cls, tb_max_entries(pl, nb, shots)) <= (size_t)smemMax;
+    }
+    // Marching tiles for devices too dense for the preferred ones: the widest of at least `strips` strips and
+    // `chunks` chunks that holds them (the smallest holds a device on each of its points).
+    bool tb_dense_plan(int nb, int cls, const aio_shot* shots, int strips, int chunks, TBPlan& out) const {
+        for (int ns = strips; ns <= std::max(strips, g.nzi / 24); ns *= 2)
+            for (int nc = chunks; nc <= std::max(chunks, g.nxi); nc *= 2) {
+                out = tb_make_plan(ns, nc);
+                if (tb_occupancy(out, cls, tb_smem(out, cls, tb_max_entries(out, nb, shots))) >= 1) return true;
+            }
+        return false;
+    }
+    // What the nonlinear adjoint and sub > 4 take on the per-fine-step stepper, which holds less per shot and
+    // any number of devices anywhere: waves that one shot's launches of four steps would not fit. (1500 devices
+    // fit a small tile wherever they are: 68 bytes each of its 227 KB.)
+    bool tb_holds(int nShots, const aio_shot* shots, bool wavefield, bool image, std::initializer_list<int> classes) const {
+        if (g.isz >= (1LL << 31) || tb_wave_capacity(nShots, shots, wavefield, image) < 1) return false;
+        TBPlan pl;
+        for (int s = 0; s < nShots; s++)
+            if (shots[s].nSourcesReg + shots[s].nReceiversReg > 1500)
+                for (int cls : classes)
+                    if (!tb_dense_plan(1, cls, shots + s, std::max(1, g.nzi / 24), g.nxi, pl)) return false;
+        return true;
+    }
+    bool tb_runs(int nShots, const aio_shot* shots, bool wavefield, bool image, std::initializer_list<int> classes) const {
+        return tb_steps() && (!tb_any_sub() || tb_holds(nShots, shots, wavefield, image, classes));
+    }
+
     // Measured autotuning of a class's plan for waves of nb shots (chunkColumns == 0): the dozen
     // candidates of the smallest modelled time are timed on an idempotent launch of interval 0
     // (the last interval for ADJ): it reads one state set and overwrites the other, the stored slice
     // 0 and the partial sums; the fastest is kept for the context and shared with the process.
     void tb_tune(int nb, const aio_shot* shots, int cls) {
-        if (P.chunkColumns != 0 || tbTuned.count(8 * nb + cls)) return;
+        auto known = tbTuned.find(8 * nb + cls);
+        if (known != tbTuned.end()) {
+            if (tb_fits(known->second, nb, cls, shots)) return;
+            tbTuned.erase(known);  // (tuned for fewer devices)
+        }
+        if (P.chunkColumns > 0) {
+            const TBPlan forced = tb_plan_c(nb, cls);
+            if (!tb_fits(forced, nb, cls, shots)) {
+                TBPlan pl;
+                require(tb_dense_plan(nb, cls, shots, forced.nStrips, forced.nChunks, pl), "blocked stepper: too many sparse devices inside one tile");
+                tbTuned[8 * nb + cls] = pl;
+            }
+            return;
+        }
         if (tb_take_shared(nb, cls, shots)) return;
         // device counts enter the candidates' shared memory: those of a mid-sized tile, then checked
         // exactly per candidate
@@ -1238,13 +1296,10 @@ struct Context {
             if (tb_occupancy(pl, cls, tb_smem(pl, cls, tb_max_entries(pl, nb, shots))) >= 1) cand.push_back(pl);
         for (const TBPlan& pl : tb_candidates(nb, cls, TBEntries{}, 16))
             if (tb_occupancy(pl, cls, tb_smem(pl, cls, tb_max_entries(pl, nb, shots))) >= 1) cand.push_back(pl);
-        if (cand.empty()) {  // devices too dense for those: the widest tile that holds its devices
-            for (int ns = 1; ns <= std::max(1, g.nzi / 24) && cand.empty(); ns *= 2)
-                for (int nc = 1; nc <= g.nxi && cand.empty(); nc *= 2) {
-                    const TBPlan pl = tb_make_plan(ns, nc);
-                    if (tb_occupancy(pl, cls, tb_smem(pl, cls, tb_max_entries(pl, nb, shots))) >= 1) cand.push_back(pl);
-                }
-            require(!cand.empty(), "blocked stepper: too many sparse devices inside one tile");
+        const bool dense = cand.empty();
+        if (dense) {
+            cand.resize(1);
+            require(tb_dense_plan(nb, cls, shots, 1, 1, cand[0]), "blocked stepper: too many sparse devices inside one tile");
         }
         cudaEvent_t e0, e1;
         AIO_CK(cudaEventCreate(&e0));
@@ -1297,8 +1352,7 @@ struct Context {
             const TBLists ml = tb_lists(pl, nb, shots, src ? 1 : (recv ? 2 : 0), record ? 1 : 0);
             tb_zero(nb, false);
             // (the heavy class's FP32 sources: whatever the stored wavefield's memory holds, as FP32 slices)
-            const bool dense = cls == TB_HEAVY || cls == TB_DENSE;
-            const int slices = dense ? (wbytes() == 4 ? g.nts : g.nts / 2) : 0;
+            const int slices = cls == TB_HEAVY || cls == TB_DENSE ? (wbytes() == 4 ? g.nts : g.nts / 2) : 0;
             tb_desc(nb, src, recv, record, cls == TB_NLC || cls == TB_NLAC ? nullptr : tbW.p, slices,
                     cls == TB_DENSE ? tbR.as<float>() : nullptr, TB_RING, din.data());
             KMArgs a = tb_args(pl, ml, nullptr);
@@ -1335,8 +1389,9 @@ struct Context {
         kernels = saveKernels;
         profEvery = saveProf;
         tbTuned[8 * nb + cls] = best;
+        if (dense) return;  // (not for contexts with fewer devices)
         std::lock_guard<std::mutex> lk(shared_plans_mu());
-        shared_plans()[shared_plan_key(8 * nb + cls)] = best;
+        shared_plans().emplace(shared_plan_key(8 * nb + cls), best);
     }
     // Per-CTA sparse lists of every shot of a wave. inj: 0 none, 1 sources, 2 receivers
     // (over the CTA's recomputed halo region); rec: 0 none, 1 receivers, 2 sources recorded (output region). Entries are
@@ -2292,7 +2347,7 @@ struct Context {
     // wavefield, :310-395 — only a batch of one shot returns it).
     void nonlinear_forward(int nShots, const aio_shot* shots, int mem, float* wavefieldOut) {
         begin_call();
-        if (tb_steps() && !wavefieldOut) return nonlinear_forward_tb(nShots, shots, mem);
+        if (!wavefieldOut && tb_runs(nShots, shots, false, false, {TB_NLC})) return nonlinear_forward_tb(nShots, shots, mem);
         Needs n;
         n.nWavefields = wavefieldOut ? 1 : 0;
         for (int s0 = 0; s0 < nShots;) {
@@ -2309,7 +2364,8 @@ struct Context {
     // Nonlinear adjoint (F/src/nonlinearShotsGpuFunctions.cu:579-652 / :653-737).
     void nonlinear_adjoint(int nShots, const aio_shot* shots, int mem, float* wavefieldOut) {
         begin_call();
-        const bool blocked = tb_steps() && !wavefieldOut && sources_move(nShots, shots);
+        const bool blocked = tb_steps() && !wavefieldOut && sources_move(nShots, shots) &&
+                             tb_holds(nShots, shots, false, false, {TB_NLAC});
         Needs n;
         n.nWavefields = wavefieldOut ? 1 : 0;
         for (int s0 = 0; s0 < nShots;) {
@@ -2353,9 +2409,9 @@ struct Context {
     }
 
 
-    // Wave sizing for the blocked stepper: per shot 4 state + 2 partial slices,
+    // Wave sizing for the blocked stepper: per shot 4 state + 2 (sub > 4: 4) partial slices,
     // the stored wavefield, an FP64 image, traces.
-    int tb_wave_size(int nShots, const aio_shot* shots, bool wavefield, bool image) {
+    long long tb_wave_capacity(int nShots, const aio_shot* shots, bool wavefield, bool image) const {
         int maxSrc = 1, maxRec = 1;
         for (int s = 0; s < nShots; s++) {
             maxSrc = std::max(maxSrc, shots[s].nSourcesReg);
@@ -2366,7 +2422,10 @@ struct Context {
                         (image ? g.isz * 8LL : 0) + (long long)maxSrc * g.ntw * 4 + 2LL * maxRec * g.nts * 4 +
                         2 * g.hsz * 4 + 2 * g.isz * 4 + (1 << 16);
         long long shared = 4LL * g.isz * 4 + (64LL << 20);
-        long long cap = (budget - shared) / per;
+        return (budget - shared) / per;
+    }
+    int tb_wave_size(int nShots, const aio_shot* shots, bool wavefield, bool image) {
+        const long long cap = tb_wave_capacity(nShots, shots, wavefield, image);
         require(cap >= 1, "device memory budget cannot hold one shot for this operator");
         return balanced_wave(cap, nShots);
     }
@@ -2438,7 +2497,7 @@ struct Context {
     void born_adjoint_shots(float* const* images, int nShots, const aio_shot* shots, int mem) {
         begin_call();
         for (int s = 0; s < nShots; s++) require(images && images[s], "per-shot image output is NULL");
-        if (tb_steps()) return born_adjoint_tb(nullptr, 0, nShots, shots, mem, images);
+        if (tb_runs(nShots, shots, true, true, {TB_LIGHT, TB_RECV})) return born_adjoint_tb(nullptr, 0, nShots, shots, mem, images);
         for (int s = 0; s < nShots; s++) born_adjoint(images[s], 0, 1, shots + s, mem);
     }
 
@@ -2462,7 +2521,7 @@ struct Context {
     // Born forward (F/src/BornShotsGpuFunctions.cu:260-388).
     void born_forward(const float* model, int nShots, const aio_shot* shots, int mem) {
         begin_call();
-        if (tb_steps()) return born_forward_tb(model, nShots, shots, mem);
+        if (tb_runs(nShots, shots, true, false, {TB_LIGHT, TB_HEAVY})) return born_forward_tb(model, nShots, shots, mem);
         Needs n;
         n.nWavefields = 1;
         n.ss = true;
@@ -2486,7 +2545,7 @@ struct Context {
     // summed on the device.
     void born_adjoint(float* modelOut, int add, int nShots, const aio_shot* shots, int mem) {
         begin_call();
-        if (tb_steps()) return born_adjoint_tb(modelOut, add, nShots, shots, mem);
+        if (tb_runs(nShots, shots, true, true, {TB_LIGHT, TB_RECV})) return born_adjoint_tb(modelOut, add, nShots, shots, mem);
         Needs n;
         n.nWavefields = 1;
         n.nImg = 1;

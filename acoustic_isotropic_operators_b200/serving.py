@@ -89,7 +89,7 @@ def shot_bytes(req: Request, wavefield_bytes: int = 4) -> int:
     g = req.grid
     isz, hsz = _slices(g)
     wavefield = req.op != "nonlinear_forward"
-    b = 6 * isz * 4 + 2 * hsz * 4 + 2 * isz * 4 + (1 << 16)
+    b = (8 if g.sub > 4 else 6) * isz * 4 + 2 * hsz * 4 + 2 * isz * 4 + (1 << 16)
     if wavefield:
         b += g.nts * isz * wavefield_bytes
         if wavefield_bytes == 2:

@@ -88,3 +88,50 @@ def test_devices_everywhere(sub):
     np.testing.assert_array_equal(out[0][0][0], out[0][0][-1])
     for a, b in zip(*out):
         assert rel_l2(a, b) < 2e-5
+
+
+@pytest.mark.parametrize("chunk", [0, 200])
+def test_plans_follow_the_devices(chunk):
+    """A plan timed (or forced) for few devices gives way to smaller tiles when a later call's do not fit."""
+    import orc
+    from acoustic_isotropic_operators_b200.batch import Context, Shot
+    c = make_case(seed=4, nzi=210, nxi=200, nts=8, sub=4, minPad=6, nshots=1, vmin=1500.0, vmax=1900.0)
+    s = c.scheme
+    k = orc.constants(s, c.vel, dtype=np.float32)
+    block = np.array([ix * s.nz + iz for ix in range(60, 160) for iz in range(60, 130)], np.int32)
+    # the source inside the block: 40 points away what arrives in 28 steps is subnormal (10 stencil hops of
+    # about 1e-4 each), where FP32 results differ by their last bits, 1e-3 of the value
+    src = block[3535:3536]
+    sig = c.sig[0][:1]
+    out = []
+    for a in (dict(chunk_columns=chunk), dict(stepper="fine")):
+        ctx = Context(s.nz, s.nx, s.nts, s.dts, s.sub, s.dz, s.dx, s.minPad, k["v2"], k["rs"], **a)
+        res = []
+        for pos in (block[3600:3603], block, block[3600:3603]):
+            data = (np.random.default_rng(2).standard_normal((len(pos), s.nts)) * 1e-2).astype(np.float32)
+            res += [ctx.nonlinear_forward([Shot(src, pos, sig)])[0].copy(),
+                    ctx.nonlinear_adjoint([Shot(src, pos, None, data)])[0].copy(),
+                    ctx.born_adjoint([Shot(src, pos, sig, data)]).copy()]
+        out.append(res)
+        ctx.close()
+    for a, b in zip(*out):
+        assert rel_l2(a, b) < 2e-5
+
+
+def test_small_budgets_take_fine_steps():
+    """The nonlinear adjoint and sub > 4 fall back to the per-fine-step stepper (same bits) where a wave of
+    the interval steppers would not fit the budget; at sub = 4 the forward is refused, as it always was."""
+    from acoustic_isotropic_operators_b200._capi import AioError
+    for sub in (4, 6):
+        c, blocked, fine = _pair(61, 50, sub, 0, 1)
+        blocked.set_budget(40 << 20)  # (below the 64 MiB a blocked wave sets aside)
+        data = [c.rng.standard_normal((len(r), c.scheme.nts)).astype(np.float32) for r in c.rec_pos]
+        np.testing.assert_array_equal(blocked.nonlinear_adjoint(_shots(c, data))[0], fine.nonlinear_adjoint(_shots(c, data))[0])
+        if sub == 4:
+            with pytest.raises(AioError):
+                blocked.nonlinear_forward(_shots(c))
+        else:
+            np.testing.assert_array_equal(blocked.nonlinear_forward(_shots(c))[0], fine.nonlinear_forward(_shots(c))[0])
+            np.testing.assert_array_equal(blocked.born_adjoint(_shots(c, data)), fine.born_adjoint(_shots(c, data)))
+        blocked.close()
+        fine.close()
