@@ -1794,19 +1794,7 @@ struct Context {
         tb_desc(nb, false, true, false, tbW.p, 0, tbR.as<float>(), LAG_K);
         KMArgs a = tb_args(pl, ml, nullptr);
         const long long mSt = (long long)g.nExt * g.isz;
-        const int nP = LAG_NP;
-        const size_t lagSmem = (size_t)lag_window_len(g.hExt) * nP * 4;
-        static int lagAttr = -1;
-        if (lagAttr != dev) {
-            AIO_CK(cudaFuncSetAttribute(k_img_lag_block<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            AIO_CK(cudaFuncSetAttribute(k_img_lag_block<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            AIO_CK(cudaFuncSetAttribute(k_img_lag_block<double, TBW_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            AIO_CK(cudaFuncSetAttribute(k_img_lag_block<float, TBW_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            AIO_CK(cudaFuncSetAttribute(k_img_lag_block<double, TBW_F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            AIO_CK(cudaFuncSetAttribute(k_img_lag_block<float, TBW_F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            lagAttr = dev;
-        }
-        require(offsets() || lagSmem <= 200 * 1024, "extension too long for the blocked lag imaging");
+        if (!offsets()) require_lags(g.hExt);
         auto image = [&](int tlo, int thi) {
             if (offsets()) {
                 // subsurface offsets (BornOffsetShotsAdjGpu, F/src/BornExtShotsGpuFunctions.cu:1848-1990):
@@ -1823,24 +1811,7 @@ struct Context {
                 kcheck();
                 return;
             }
-            const dim3 grid((unsigned)((g.isz + nP - 1) / nP), nb);
-            const long long rSt = (long long)LAG_K * g.isz;
-            const float* sc = f16() ? tbWscale.as<float>() : nullptr;
-#define AIO_LAG_IMG(ACC, WP)                                                                                          \
-    k_img_lag_block<ACC, WP><<<grid, nP, lagSmem, st>>>(img.as<ACC>(), mSt, tbR.as<float>(), rSt, LAG_K, tbW.p, wfSt(), \
-                                                        g.isz, tlo, thi, g.nts, g.hExt, g.nExt, 1, sc)
-            if (P.wavefieldPrecision == AIO_WFLD_BF16) {
-                if (P.imageFp64) AIO_LAG_IMG(double, TBW_BF16);
-                else AIO_LAG_IMG(float, TBW_BF16);
-            } else if (f16()) {
-                if (P.imageFp64) AIO_LAG_IMG(double, TBW_F16);
-                else AIO_LAG_IMG(float, TBW_F16);
-            } else {
-                if (P.imageFp64) AIO_LAG_IMG(double, TBW_F32);
-                else AIO_LAG_IMG(float, TBW_F32);
-            }
-#undef AIO_LAG_IMG
-            kcheck();
+            lag_image(nb, mSt, tbR.as<float>(), LAG_K, tbW.p, src_wp(), tlo, thi, g.hExt, g.nExt, 1);
         };
         for (int L = 0; L < g.nts - 1; L++) {
             tb_step(a, L, true);
@@ -1865,50 +1836,20 @@ struct Context {
         tb_zero(nb, false);
         tb_desc(nb, false, false, true, tbSS.p, ring);
         KMArgs a = tb_args(pl, ml, nullptr);
-        const int nP = LAG_NP;
-        const size_t lagSmem = (size_t)lag_window_len(g.hExt) * nP * 4;
-        static int ssAttr = -1;
-        if (ssAttr != dev) {
-            AIO_CK(cudaFuncSetAttribute(k_ss_lag_block<TBW_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            AIO_CK(cudaFuncSetAttribute(k_ss_lag_block<TBW_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            AIO_CK(cudaFuncSetAttribute(k_ss_lag_block<TBW_F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            ssAttr = dev;
-        }
-        require(offsets() || lagSmem <= 200 * 1024, "extension too long for the blocked lag imaging");
+        if (!offsets()) require_lags(g.hExt);
         auto sources = [&](int tlo) {
             const int thi = std::min(tlo + LAG_K - 1, g.nts - 1);
             if (offsets()) {
-                // subsurface offsets (imagingOffsetFwdGpu + scaleSecondarySourceFd): one slice per
-                // sample, formed into the zeroed ring slots of the block
-                const long long rSt = (long long)ring * g.isz;
-                AIO_CK(cudaMemset2DAsync(tbSS.as<float>() + (long long)(tlo % ring) * g.isz, (size_t)rSt * 4, 0,
-                                         (size_t)(thi - tlo + 1) * g.isz * 4, nb, st));
-                const float* Fs = F ? F : tbW.as<float>();
-                for (int t = tlo; t <= thi; t++)
-                    k_img_offset_fwd<<<ew_grid(nb, g.isz), 256, 0, st>>>(
-                        tbSS.as<float>() + (long long)(t % ring) * g.isz, rSt, ext, 0, Fs + (long long)t * g.isz,
-                        wfSt(), v2p(), g.isz, g.ip, g.nxi, g.hExt);
+                // subsurface offsets (imagingOffsetFwdGpu + scaleSecondarySourceFd)
+                k_img_offset_fwd_block<<<dim3((unsigned)((g.ip + 127) / 128), (unsigned)((g.nxi + 2 * OFF_J - 1) / (2 * OFF_J) * 2),
+                                              (unsigned)(nb * ((thi - tlo + OFF_S) / OFF_S))),
+                                         128, 0, st>>>(tbSS.as<float>(), (long long)ring * g.isz, ring, ext,
+                                                       F ? F : tbW.as<float>(), wfSt(), v2p(), g.isz, g.ip, g.nxi, g.hExt, tlo, thi);
                 kcheck();
                 return;
             }
-            const dim3 grid((unsigned)((g.isz + nP - 1) / nP), nb);
             // F (a caller's FP32 field) or the stored source wavefield in its precision
-            const int wp = F ? AIO_WFLD_FP32 : P.wavefieldPrecision;
-            const void* Ws = F ? (const void*)F : tbW.p;
-            const float* sc = (!F && f16()) ? tbWscale.as<float>() : nullptr;
-            if (wp == AIO_WFLD_BF16)
-                k_ss_lag_block<TBW_BF16><<<grid, nP, lagSmem, st>>>(tbSS.as<float>(), (long long)ring * g.isz, ring, ext,
-                                                                    Ws, wfSt(), g.isz, tlo, thi, g.nts, g.hExt, g.nExt,
-                                                                    1, sc);
-            else if (wp == AIO_WFLD_FP16)
-                k_ss_lag_block<TBW_F16><<<grid, nP, lagSmem, st>>>(tbSS.as<float>(), (long long)ring * g.isz, ring, ext,
-                                                                   Ws, wfSt(), g.isz, tlo, thi, g.nts, g.hExt, g.nExt,
-                                                                   1, sc);
-            else
-                k_ss_lag_block<TBW_F32><<<grid, nP, lagSmem, st>>>(tbSS.as<float>(), (long long)ring * g.isz, ring, ext,
-                                                                   Ws, wfSt(), g.isz, tlo, thi, g.nts, g.hExt, g.nExt,
-                                                                   1, sc);
-            kcheck();
+            lag_sources(nb, ring, ext, F ? (const void*)F : tbW.p, F ? (int)TBW_F32 : src_wp(), tlo, thi, 1);
         };
         for (int its = 0; its < g.nts - 1; its++) {
             if (its == 0) sources(0);
@@ -1995,68 +1936,55 @@ struct Context {
         return P.wavefieldPrecision == AIO_WFLD_BF16 ? TBW_BF16 : (P.wavefieldPrecision == AIO_WFLD_FP16 ? TBW_F16 : TBW_F32);
     }
 
-    void tb_lag_attr() {
-        static int lagDev = -1;
-        if (lagDev == dev) return;
-        const int b = 200 * 1024;
-        AIO_CK(cudaFuncSetAttribute(k_img_lag_block<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-        AIO_CK(cudaFuncSetAttribute(k_img_lag_block<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-        AIO_CK(cudaFuncSetAttribute(k_img_lag_block<double, TBW_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-        AIO_CK(cudaFuncSetAttribute(k_img_lag_block<float, TBW_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-        AIO_CK(cudaFuncSetAttribute(k_img_lag_block<double, TBW_F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-        AIO_CK(cudaFuncSetAttribute(k_img_lag_block<float, TBW_F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-        AIO_CK(cudaFuncSetAttribute(k_ss_lag_block<TBW_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-        AIO_CK(cudaFuncSetAttribute(k_ss_lag_block<TBW_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-        AIO_CK(cudaFuncSetAttribute(k_ss_lag_block<TBW_F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, b));
-        lagDev = dev;
+    // (a limit of earlier kernels' shared memory)
+    void require_lags(int hExt) const { require(hExt <= 92, "extension too long for the blocked lag imaging"); }
+    // f(precision, sign) with both as constants
+    template <class F>
+    static void lag_form(int wp, int sign, F&& f) {
+        auto of = [&](auto w) {
+            if (sign > 0) f(w, std::integral_constant<int, 1>());
+            else f(w, std::integral_constant<int, -1>());
+        };
+        if (wp == TBW_BF16) of(std::integral_constant<int, TBW_BF16>());
+        else if (wp == TBW_F16) of(std::integral_constant<int, TBW_F16>());
+        else of(std::integral_constant<int, TBW_F32>());
     }
-    size_t tb_lag_smem(int hExt) const {
-        const size_t b = (size_t)lag_window_len(hExt) * LAG_NP * 4;
-        require(b <= 200 * 1024, "extension too long for the blocked lag imaging");
-        return b;
+    // secondary sources of the samples [tlo, thi] into the ring tbSS
+    void lag_sources(int nb, int ring, const float* ext, const void* W, int wp, int tlo, int thi, int sign) {
+        const dim3 grid((unsigned)((g.isz + LAG_NP - 1) / LAG_NP), nb);
+        lag_form(wp, sign, [&](auto w, auto sg) {
+            k_ss_lag_block<decltype(w)::value, decltype(sg)::value><<<grid, LAG_NP, 0, st>>>(
+                tbSS.as<float>(), (long long)ring * g.isz, ring, ext, W, wfSt(), g.isz, tlo, thi, g.nts, g.hExt, g.nExt,
+                tbWscale.as<float>());
+        });
+        kcheck();
+    }
+    // image the samples [tlo, thi] of the ring R against the field W
+    void lag_image(int nb, long long mSt, const float* R, int ring, const void* W, int wp, int tlo, int thi, int hE, int nE,
+                   int sign) {
+        const dim3 grid((unsigned)((g.isz + LAG_NP - 1) / LAG_NP), nb);
+        lag_form(wp, sign, [&](auto w, auto sg) {
+            if (P.imageFp64)
+                k_img_lag_block<double, decltype(w)::value, decltype(sg)::value><<<grid, LAG_NP, 0, st>>>(
+                    img.as<double>(), mSt, R, (long long)ring * g.isz, ring, W, wfSt(), g.isz, tlo, thi, g.nts, hE, nE,
+                    tbWscale.as<float>());
+            else
+                k_img_lag_block<float, decltype(w)::value, decltype(sg)::value><<<grid, LAG_NP, 0, st>>>(
+                    img.as<float>(), mSt, R, (long long)ring * g.isz, ring, W, wfSt(), g.isz, tlo, thi, g.nts, hE, nE,
+                    tbWscale.as<float>());
+        });
+        kcheck();
     }
     // secondary sources of the coarse steps [tlo, thi] into the ring tbSS
     void tb_ss_block(int nb, const TBSrc& src, int tlo, int thi) {
-        tb_lag_attr();
-        const int nP = LAG_NP;
-        const dim3 grid((unsigned)((g.isz + nP - 1) / nP), nb);
-        const size_t sm = tb_lag_smem(g.hExt);
-        const long long rSt = (long long)TB_RING * g.isz;
-        float* ss = tbSS.as<float>();
-        if (src.wp == TBW_BF16)
-            k_ss_lag_block<TBW_BF16><<<grid, nP, sm, st>>>(ss, rSt, TB_RING, src.ext, src.F, wfSt(), g.isz, tlo, thi,
-                                                           g.nts, g.hExt, g.nExt, src.sign);
-        else if (src.wp == TBW_F16)
-            k_ss_lag_block<TBW_F16><<<grid, nP, sm, st>>>(ss, rSt, TB_RING, src.ext, src.F, wfSt(), g.isz, tlo, thi,
-                                                          g.nts, g.hExt, g.nExt, src.sign, tbWscale.as<float>());
-        else
-            k_ss_lag_block<TBW_F32><<<grid, nP, sm, st>>>(ss, rSt, TB_RING, src.ext, src.F, wfSt(), g.isz, tlo, thi,
-                                                          g.nts, g.hExt, g.nExt, src.sign);
-        kcheck();
+        require_lags(g.hExt);
+        lag_sources(nb, TB_RING, src.ext, src.F, src.wp, tlo, thi, src.sign);
     }
     // image the samples [tlo, thi] of the ring tbR against out.imgF
     void tb_img_block(int nb, const TBOut& out, int tlo, int thi) {
-        tb_lag_attr();
-        const int nP = LAG_NP, nE = out.lag ? g.nExt : 1, hE = out.lag ? g.hExt : 0;
-        const dim3 grid((unsigned)((g.isz + nP - 1) / nP), nb);
-        const long long mSt = (long long)nE * g.isz, rSt = (long long)TB_RING * g.isz;
-        const size_t sm = tb_lag_smem(hE);
-        const float* R = tbR.as<float>();
-        const float* sc = out.wp == TBW_F16 ? tbWscale.as<float>() : nullptr;
-#define AIO_TB_IMG(ACC, WP)                                                                                         \
-    k_img_lag_block<ACC, WP><<<grid, nP, sm, st>>>(img.as<ACC>(), mSt, R, rSt, TB_RING, out.imgF, wfSt(), g.isz, tlo, \
-                                                   thi, g.nts, hE, nE, out.sign, sc)
-        if (P.imageFp64) {
-            if (out.wp == TBW_BF16) AIO_TB_IMG(double, TBW_BF16);
-            else if (out.wp == TBW_F16) AIO_TB_IMG(double, TBW_F16);
-            else AIO_TB_IMG(double, TBW_F32);
-        } else {
-            if (out.wp == TBW_BF16) AIO_TB_IMG(float, TBW_BF16);
-            else if (out.wp == TBW_F16) AIO_TB_IMG(float, TBW_F16);
-            else AIO_TB_IMG(float, TBW_F32);
-        }
-#undef AIO_TB_IMG
-        kcheck();
+        const int nE = out.lag ? g.nExt : 1, hE = out.lag ? g.hExt : 0;
+        require_lags(hE);
+        lag_image(nb, (long long)nE * g.isz, tbR.as<float>(), TB_RING, out.imgF, out.wp, tlo, thi, hE, nE, out.sign);
     }
 
     // Forward-time dense pass (fwd_dense_pass on the blocked stepper, TB_SCATW):

@@ -13,6 +13,7 @@
 // stores each level once (damped once) and applies the second damping factor
 // when it reads p_old, which produces the same values with one store per point.
 #pragma once
+#include <type_traits>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -289,6 +290,77 @@ __global__ void k_img_offset_fwd(float* ss, long long ssSt, const float* m, long
         ss[i] = acc * v2[i];
     }
 }
+// imagingOffsetFwdGpu for the samples tlo..thi, written to ring slots t % ring: ss_t(x) = v2(x) sum_s
+// m_{s+h}(x-s) W_t(x-2s). A thread forms OFF_S samples of OFF_J columns x0, x0 + 2, ...: with s, the
+// columns that they read move by one of these steps, so that one new column is loaded per s and sample, and
+// each m once for all samples: per term 0.36 loads from L2, which bound a launch per sample that had 2. One B200,
+// 21 offsets, 2 shots of 512 x 1312 points, 32 samples: 0.44 ms (1.35 ms by samples; 0.76 without the loads
+// a step ahead, where every m of a step cost a latency of its own).
+constexpr int OFF_J = 4, OFF_S = 8;
+__global__ void __launch_bounds__(128, 4) k_img_offset_fwd_block(float* __restrict__ ss, long long ssSt, int ring,
+                                                              const float* __restrict__ m, const float* __restrict__ W,
+                                                              long long WSt, const float* __restrict__ v2, long long isz,
+                                                              int ip, int nxi, int hExt, int tlo, int thi) {
+    const int z = blockIdx.x * 128 + threadIdx.x, x0 = (int)(blockIdx.y >> 1) * 2 * OFF_J + (int)(blockIdx.y & 1);
+    const int nT = (thi - tlo + OFF_S) / OFF_S, b = blockIdx.z / nT, t0 = tlo + (blockIdx.z % nT) * OFF_S;
+    if (z >= ip || x0 >= nxi) return;
+    ss += b * ssSt + z;
+    m += z;
+    W += b * WSt + (long long)t0 * isz + z;
+    v2 += z;
+    const int nk = min(thi - t0 + 1, OFF_S);
+    float acc[OFF_J][OFF_S], w[OFF_J][OFF_S];  // w: column j's of step n in place (j - n) mod OFF_J
+    auto column = [&](float(&o)[OFF_S], int x) {
+        const bool in = x >= 0 && x < nxi;
+#pragma unroll
+        for (int k = 0; k < OFF_S; k++) o[k] = in && k < nk ? __ldg(W + (long long)k * isz + (long long)x * ip) : 0.f;
+    };
+#pragma unroll
+    for (int j = 0; j < OFF_J; j++) {
+        column(w[j], x0 + 2 * j + 2 * hExt);
+#pragma unroll
+        for (int k = 0; k < OFF_S; k++) acc[j][k] = 0.f;
+    }
+    // (a step's model points and the next one's column are loaded a step ahead of their use)
+    auto model = [&](int j, int s) { return x0 + 2 * j - s; };
+    auto inside = [&](int j, int s) {
+        return s <= hExt && x0 + 2 * j < nxi && model(j, s) >= hExt && model(j, s) < nxi - hExt;
+    };
+    auto coef = [&](int j, int s) { return inside(j, s) ? __ldg(m + (long long)(s + hExt) * isz + (long long)model(j, s) * ip) : 0.f; };
+    float c[OFF_J];
+#pragma unroll
+    for (int j = 0; j < OFF_J; j++) c[j] = coef(j, -hExt);
+    for (int s0 = -hExt; s0 <= hExt; s0 += OFF_J)
+#pragma unroll
+        for (int n = 0; n < OFF_J; n++) {
+            const int s = s0 + n;
+            float cn[OFF_J], next[OFF_S];
+#pragma unroll
+            for (int j = 0; j < OFF_J; j++) cn[j] = coef(j, s + 1);
+            column(next, s < hExt ? x0 - 2 * (s + 1) : -1);
+#pragma unroll
+            for (int j = 0; j < OFF_J; j++) {
+                const bool in = inside(j, s);
+#pragma unroll
+                for (int k = 0; k < OFF_S; k++) {
+                    const float a = fmaf(c[j], w[(j - n + OFF_J) % OFF_J][k], acc[j][k]);
+                    acc[j][k] = in ? a : acc[j][k];
+                }
+                c[j] = cn[j];
+            }
+#pragma unroll
+            for (int k = 0; k < OFF_S; k++) w[OFF_J - 1 - n][k] = next[k];
+        }
+#pragma unroll
+    for (int j = 0; j < OFF_J; j++) {
+        const int x = x0 + 2 * j;
+        if (x >= nxi) break;
+        const float v = __ldg(v2 + (long long)x * ip);
+#pragma unroll
+        for (int k = 0; k < OFF_S; k++)
+            if (k < nk) ss[(long long)((t0 + k) % ring) * isz + (long long)x * ip] = acc[j][k] * v;
+    }
+}
 // imagingOffsetTomoAdjGpu (:460-476): ss(x) += sum_s m_{s+h}(x+s) R(x+2s) v2(x+2s) over the offsets
 // whose model point x+s lies in [h, nxi-h). With v2Out (U-form receiver wavefield, R = v2 R_ref
 // already, v2Rec = nullptr): ss(x) = v2(x) * (ss(x) + sum_s m_{s+h}(x+s) R(x+2s)).
@@ -372,34 +444,19 @@ __global__ void k_img_offset_block(Acc* img, long long mSt, const float* R, long
 //   img[e] += sum_{t = tlo..thi} R(t) * W[t - sign 2(e-h)]   over 0 <= t - sign 2(e-h) < nts,
 // the same (t, e) pairs as the reference's truncating-division lag bounds (nExt = 1, hExt = 0:
 // the zero-lag imagingAdjGpu, :318-325). R(t) lives in a ring of rRing slices (slot t % rRing).
-// Each thread owns one point: its R samples are held in registers and the W slices
-// tlo-2h .. tlo+LAG_K-1+2h of the block in shared memory (own column only, no barrier; zero
+// Each thread owns one point: its R samples are held in registers and the W samples
+// tlo-2h .. tlo+LAG_K-1+2h of the block pass through a window of registers (LagWindow; zero
 // outside [0, nts), so every (t, e) term is formed without bounds tests and the terms outside
 // the reference's bounds add exact zeros), so W is read once per block instead of once per lag,
 // and the image once per block instead of once per sample. Global loads are issued in batches:
 // the kernels are latency bound otherwise.
 constexpr int LAG_K = 32;
 constexpr int LAG_B = 8;
-constexpr int LAG_NP = 128;  // threads per block (points), a compile-time shared-memory stride
-__host__ __device__ constexpr int lag_window_len(int hExt) { return LAG_K + 4 * hExt; }
-// Sample tau of a stored wavefield at element idx: FP32, BF16, or FP16 in units of the slice's
-// scale sc[tau] (the stored source wavefield of aio_tb.cuh).
-template <int WP>
-__device__ __forceinline__ float lag_wsample(const void* __restrict__ W, long long idx, const float* __restrict__ sc,
-                                             int tau) {
-    if (WP == TBW_F32) return __ldg(reinterpret_cast<const float*>(W) + idx);
-    const unsigned short u = __ldg(reinterpret_cast<const unsigned short*>(W) + idx);
-    if (WP == TBW_BF16) return __bfloat162float(__ushort_as_bfloat16(u));
-    return __half2float(__ushort_as_half(u)) * __ldg(sc + tau);
-}
-// W slices tlo-2h .. of point p into this thread's shared column, zero outside [0, nts). The
-// column holds consecutive samples in pairs (one float2 per pair): every lag offset 2h - 2(e-h)
-// is even, so sample pairs (k, k+1) of any lag are one aligned float2 and the inner products
-// run on paired FP32 instructions. W is stored in FP32, BF16 or FP16 with per-slice scales sc.
+constexpr int LAG_NP = 128;  // threads per block (points)
 //
 // 16-bit samples: the two lanes of a point pair (p even, p + 1; slices are a whole number of
 // warps, isz % 32 == 0, so both lanes always run) share 32-bit loads. For each sample pair
-// (k, k+1) the even lane loads the pair's word of slice k, the odd lane the word of slice k+1,
+// the even lane loads the pair's word of the first slice, the odd lane the word of the second,
 // and one shuffle hands each lane the other word: every lane then holds its own point's two
 // samples. Half the load instructions of one 16-bit load per sample, four bytes per lane.
 template <int WP>
@@ -408,72 +465,101 @@ __device__ __forceinline__ float lag_half(unsigned word, bool high) {
     if (WP == TBW_BF16) return __bfloat162float(__ushort_as_bfloat16(u));
     return __half2float(__ushort_as_half(u));
 }
-template <int WP = TBW_F32>
-__device__ __forceinline__ void lag_window(float2* W2, const void* __restrict__ W, const float* __restrict__ sc,
-                                           long long isz, long long p, int tlo, int hExt, int nts) {
-    const int n = lag_window_len(hExt), t0 = tlo - 2 * hExt;
-    if constexpr (WP == TBW_F32) {
-        for (int k0 = 0; k0 < n; k0 += 2 * LAG_B) {
-            float v[2 * LAG_B];
+// The window of a point's samples that a block of lags multiplies, held in registers. Every lag offset
+// 2(e-h) is even, so a lag's LAG_K samples are LAG_K/2 pairs and the products run on paired FP32
+// instructions; the next lag's are the same ones moved by one pair. Pair i of the sequence starts at sample
+// s0 + 2 SIGN i, lag e's pair kp is number e + (SIGN > 0 ? kp : LAG_K/2 - 1 - kp): per lag one new pair is
+// loaded, LAG_B at a time into the LAG_B oldest places. Pair i's place: i mod LAG_W. (The window lay in shared
+// memory before, read anew for every lag: LAG_P 8-byte reads per lag and point bound the kernels. One B200, 31
+// lags, BF16 field, 8 shots of 608 x 1600 points: an image block 1.51 -> 1.13 ms, 0.66 at the copy rate.)
+constexpr int LAG_P = LAG_K / 2, LAG_W = LAG_P + LAG_B;
+static_assert(LAG_W == 3 * LAG_B, "three groups of lags per turn of the window");
+template <int WP, int SIGN>
+struct LagWindow {
+    float2 v[LAG_W];
+    const void* W;
+    const float* sc;
+    long long isz, p;
+    int s0, nts, n;  // first pair's sample, samples, pairs of all lags
+    // pairs i0 .. i0 + LAG_B - 1, i0 mod LAG_W == I
+    template <int I>
+    __device__ __forceinline__ void load(int i0) {
+        if constexpr (WP == TBW_F32) {
 #pragma unroll
-            for (int j = 0; j < 2 * LAG_B; j++) {
-                const int tau = t0 + k0 + j;
-                v[j] = (k0 + j < n && tau >= 0 && tau < nts) ? lag_wsample<WP>(W, (long long)tau * isz + p, sc, tau)
-                                                             : 0.f;
+            for (int j = 0; j < LAG_B; j++) {
+                const int t = s0 + 2 * SIGN * (i0 + j);
+                const bool in = i0 + j < n;
+                v[(I + j) % LAG_W] = make_float2(in && t >= 0 && t < nts ? __ldg((const float*)W + (long long)t * isz + p) : 0.f,
+                                                 in && t >= -1 && t + 1 < nts ? __ldg((const float*)W + (long long)(t + 1) * isz + p) : 0.f);
             }
-#pragma unroll
-            for (int j = 0; j < 2 * LAG_B; j += 2)
-                if (k0 + j < n) W2[((k0 + j) >> 1) * LAG_NP] = make_float2(v[j], v[j + 1]);
-        }
-    } else {
-        const bool odd = (p & 1) != 0;
-        const unsigned* __restrict__ W32 = reinterpret_cast<const unsigned*>(W);
-        const long long iszw = isz >> 1, pw = p >> 1;
-        for (int k0 = 0; k0 < n; k0 += 2 * LAG_B) {
+        } else {
+            const bool odd = (p & 1) != 0;
+            const unsigned* __restrict__ W32 = reinterpret_cast<const unsigned*>(W);
+            const long long iszw = isz >> 1, pw = p >> 1;
             unsigned wv[LAG_B];
 #pragma unroll
             for (int j = 0; j < LAG_B; j++) {
-                const int k = k0 + 2 * j + (odd ? 1 : 0);  // the sample this lane loads
-                const int tau = t0 + k;
-                wv[j] = (k < n && tau >= 0 && tau < nts) ? __ldg(W32 + (long long)tau * iszw + pw) : 0u;
+                const int t = s0 + 2 * SIGN * (i0 + j) + (odd ? 1 : 0);  // the sample this lane loads
+                wv[j] = i0 + j < n && t >= 0 && t < nts ? __ldg(W32 + (long long)t * iszw + pw) : 0u;
             }
 #pragma unroll
             for (int j = 0; j < LAG_B; j++) {
                 const unsigned other = __shfl_xor_sync(0xffffffffu, wv[j], 1);
-                const int k = k0 + 2 * j;
-                if (k < n) {
-                    float va = lag_half<WP>(odd ? other : wv[j], odd);  // sample k of this point
-                    float vb = lag_half<WP>(odd ? wv[j] : other, odd);  // sample k + 1
-                    if (WP == TBW_F16) {
-                        const int ta = t0 + k;
-                        va *= (ta >= 0 && ta < nts) ? __ldg(sc + ta) : 0.f;
-                        vb *= (ta + 1 >= 0 && ta + 1 < nts) ? __ldg(sc + ta + 1) : 0.f;
-                    }
-                    W2[(k >> 1) * LAG_NP] = make_float2(va, vb);
+                float va = lag_half<WP>(odd ? other : wv[j], odd);
+                float vb = lag_half<WP>(odd ? wv[j] : other, odd);
+                if (WP == TBW_F16) {
+                    const int t = s0 + 2 * SIGN * (i0 + j);
+                    va *= t >= 0 && t < nts ? __ldg(sc + t) : 0.f;
+                    vb *= t >= -1 && t + 1 < nts ? __ldg(sc + t + 1) : 0.f;
                 }
+                v[(I + j) % LAG_W] = make_float2(va, vb);
             }
         }
     }
-}
+    // `sign` > 0: samples t - 2(e-h) of lag e (SIGN = -1), else t + 2(e-h)
+    __device__ __forceinline__ LagWindow(const void* W_, const float* sc_, long long isz_, long long p_, int tlo, int nts_,
+                                         int hExt, int nExt)
+        : W(W_), sc(sc_), isz(isz_), p(p_), s0(SIGN < 0 ? tlo + 2 * hExt + LAG_K - 2 : tlo - 2 * hExt), nts(nts_),
+          n(nExt + LAG_P - 1) {
+        load<0>(0);
+        load<LAG_B>(LAG_B);
+    }
+    // pair kp of the lag that is lag j of the group whose first pair has place ROT
+    template <int ROT>
+    __device__ __forceinline__ const float2& at(int j, int kp) const {
+        return v[(ROT + j + (SIGN > 0 ? kp : LAG_P - 1 - kp)) % LAG_W];
+    }
+    // f(e0, place) for every group of LAG_B lags, its window loaded
+    template <class Group>
+    __device__ __forceinline__ void groups(int nExt, Group&& f) {
+        for (int e0 = 0;; e0 += 3 * LAG_B) {
+            load<LAG_P>(e0 + LAG_P);
+            f(e0, std::integral_constant<int, 0>());
+            if (e0 + LAG_B >= nExt) break;
+            load<LAG_P + LAG_B>(e0 + LAG_B + LAG_P);
+            f(e0 + LAG_B, std::integral_constant<int, LAG_B>());
+            if (e0 + 2 * LAG_B >= nExt) break;
+            load<LAG_P + 2 * LAG_B>(e0 + 2 * LAG_B + LAG_P);
+            f(e0 + 2 * LAG_B, std::integral_constant<int, 2 * LAG_B>());
+            if (e0 + 3 * LAG_B >= nExt) break;
+        }
+    }
+};
 // W: stored wavefield of WSt elements per shot (FP32, or BF16 / FP16 with nts scales per shot
 // in wsc when WP says so).
-template <typename Acc, int WP = TBW_F32>
+template <typename Acc, int WP, int SIGN>
 __global__ void __launch_bounds__(LAG_NP) k_img_lag_block(Acc* __restrict__ img, long long mSt, const float* __restrict__ R,
                                                           long long rSt, int rRing, const void* __restrict__ W,
                                                           long long WSt, long long isz, int tlo, int thi, int nts,
-                                                          int hExt, int nExt, int sign,
-                                                          const float* __restrict__ wsc = nullptr) {
-    extern __shared__ float2 lag_smem2[];
+                                                          int hExt, int nExt, const float* __restrict__ wsc) {
     const int b = blockIdx.y, tid = threadIdx.x;
     const long long p = (long long)blockIdx.x * LAG_NP + tid;
     if (p >= isz) return;
     R += b * rSt;
     const void* Wb = reinterpret_cast<const char*>(W) + b * WSt * (WP == TBW_F32 ? 4 : 2);
-    const float* scb = WP == TBW_F16 ? wsc + (long long)b * nts : nullptr;
     img += b * mSt;
-    float2* W2 = lag_smem2 + tid;
-    lag_window<WP>(W2, Wb, scb, isz, p, tlo, hExt, nts);
-    float2 r2[LAG_K / 2];
+    LagWindow<WP, -SIGN> w(Wb, WP == TBW_F16 ? wsc + (long long)b * nts : nullptr, isz, p, tlo, nts, hExt, nExt);
+    float2 r2[LAG_P];
     int slot = tlo % rRing;  // ring slot of sample tlo; the block's slots follow with one wrap at most
 #pragma unroll
     for (int k = 0; k < LAG_K; k += 2) {
@@ -483,68 +569,55 @@ __global__ void __launch_bounds__(LAG_NP) k_img_lag_block(Acc* __restrict__ img,
         slot = slot + 1 == rRing ? 0 : slot + 1;
         r2[k >> 1] = make_float2(ra, rb);
     }
-    for (int e0 = 0; e0 < nExt; e0 += LAG_B) {
-        float acc[LAG_B];
-#pragma unroll
-        for (int j = 0; j < LAG_B; j++) {
-            // W index of sample k at lag e: tlo + k - sign 2(e-h), window offset 2h - sign 2(e-h)
-            const int e = min(e0 + j, nExt - 1);
-            const float2* w = W2 + ((2 * hExt - sign * 2 * (e - hExt)) >> 1) * LAG_NP;
-            float2 sum = make_float2(0.f, 0.f);  // even and odd samples of the block
-#pragma unroll
-            for (int kp = 0; kp < LAG_K / 2; kp++) sum = __ffma2_rn(r2[kp], w[kp * LAG_NP], sum);
-            acc[j] = sum.x + sum.y;
-        }
+    w.groups(nExt, [&](int e0, auto rot) {
+        constexpr int ROT = decltype(rot)::value;
         Acc old[LAG_B];
 #pragma unroll
         for (int j = 0; j < LAG_B; j++) old[j] = e0 + j < nExt ? img[(long long)(e0 + j) * isz + p] : (Acc)0;
 #pragma unroll
-        for (int j = 0; j < LAG_B; j++)
-            if (e0 + j < nExt) img[(long long)(e0 + j) * isz + p] = old[j] + (Acc)acc[j];
-    }
+        for (int j = 0; j < LAG_B; j++) {
+            if (e0 + j >= nExt) break;
+            float2 sum = make_float2(0.f, 0.f);  // even and odd samples of the block
+#pragma unroll
+            for (int kp = 0; kp < LAG_P; kp++) sum = __ffma2_rn(r2[kp], w.template at<ROT>(j, kp), sum);
+            img[(long long)(e0 + j) * isz + p] = old[j] + (Acc)(sum.x + sum.y);
+        }
+    });
 }
 
 // Secondary sources of a block of coarse steps of the time-lag extended forward
 // (imagingTimeFwdGpu, F/src/kernelsGpu.cu:337-350, at every t of the block; sign = -1 gives
 // imagingTimeTomoAdjGpu, :445-458):
 //   ss(t) = sum_e ext[e] * W[t - sign 2(e-h)]   over 0 <= t - sign 2(e-h) < nts,
-// written to a ring of ring slices (slot t % ring). One thread per point; the W slices of
-// the block live in shared memory (own column only, zero outside [0, nts)), so W is read once
-// per block, and ext once per block (lags outer, the block's samples accumulated in registers,
-// in lag order, two samples per paired instruction).
-template <int WP = TBW_F32>
+// written to a ring of ring slices (slot t % ring). One thread per point, the block's samples
+// accumulated in registers, in lag order, two samples per paired instruction.
+template <int WP, int SIGN>
 __global__ void __launch_bounds__(LAG_NP) k_ss_lag_block(float* __restrict__ ss, long long ssSt, int ring,
                                                          const float* __restrict__ ext, const void* __restrict__ W,
                                                          long long WSt, long long isz, int tlo, int thi, int nts,
-                                                         int hExt, int nExt, int sign,
-                                                         const float* __restrict__ wsc = nullptr) {
-    extern __shared__ float2 lag_smem2[];
+                                                         int hExt, int nExt, const float* __restrict__ wsc) {
     const int b = blockIdx.y, tid = threadIdx.x;
     const long long p = (long long)blockIdx.x * LAG_NP + tid;
     if (p >= isz) return;
     ss += b * ssSt;
     const void* Wb = reinterpret_cast<const char*>(W) + b * WSt * (WP == TBW_F32 ? 4 : 2);
-    const float* scb = WP == TBW_F16 ? wsc + (long long)b * nts : nullptr;
-    float2* W2 = lag_smem2 + tid;
-    lag_window<WP>(W2, Wb, scb, isz, p, tlo, hExt, nts);
-    float2 acc[LAG_K / 2];
+    LagWindow<WP, -SIGN> w(Wb, WP == TBW_F16 ? wsc + (long long)b * nts : nullptr, isz, p, tlo, nts, hExt, nExt);
+    float2 acc[LAG_P];
 #pragma unroll
-    for (int k = 0; k < LAG_K / 2; k++) acc[k] = make_float2(0.f, 0.f);
-    for (int e0 = 0; e0 < nExt; e0 += LAG_B) {
+    for (int k = 0; k < LAG_P; k++) acc[k] = make_float2(0.f, 0.f);
+    w.groups(nExt, [&](int e0, auto rot) {
+        constexpr int ROT = decltype(rot)::value;
         float x[LAG_B];
 #pragma unroll
         for (int j = 0; j < LAG_B; j++) x[j] = e0 + j < nExt ? __ldg(ext + (long long)(e0 + j) * isz + p) : 0.f;
 #pragma unroll
         for (int j = 0; j < LAG_B; j++) {
-            if (e0 + j < nExt) {
-                const int e = e0 + j;
-                const float2* w = W2 + ((2 * hExt - sign * 2 * (e - hExt)) >> 1) * LAG_NP;
-                const float2 xx = make_float2(x[j], x[j]);
+            if (e0 + j >= nExt) break;
+            const float2 xx = make_float2(x[j], x[j]);
 #pragma unroll
-                for (int kp = 0; kp < LAG_K / 2; kp++) acc[kp] = __ffma2_rn(xx, w[kp * LAG_NP], acc[kp]);
-            }
+            for (int kp = 0; kp < LAG_P; kp++) acc[kp] = __ffma2_rn(xx, w.template at<ROT>(j, kp), acc[kp]);
         }
-    }
+    });
     int slot = tlo % ring;  // ring slot of sample tlo; the block's slots follow with one wrap at most
 #pragma unroll
     for (int k = 0; k < LAG_K; k += 2) {

@@ -135,3 +135,26 @@ def test_small_budgets_take_fine_steps():
             np.testing.assert_array_equal(blocked.born_adjoint(_shots(c, data)), fine.born_adjoint(_shots(c, data)))
         blocked.close()
         fine.close()
+
+
+@pytest.mark.parametrize("extension", ["time", "offset"])
+@pytest.mark.parametrize("nExt,nzi,nxi,nts", [(1, 33, 23, 5), (3, 40, 24, 34), (9, 129, 25, 33), (17, 35, 64, 41), (19, 37, 67, 66)])
+def test_extended_blocks(nExt, nzi, nxi, nts, extension):
+    """Blocks of samples at the edges of their groups: lags around 8 and 16, samples around 32, columns around
+    8, offsets wider than the grid allows."""
+    import orc
+    from acoustic_isotropic_operators_b200.batch import Context
+    c = make_case(seed=nExt, nzi=nzi, nxi=nxi, nts=nts, sub=4, minPad=6, nshots=2, vmin=1500.0, vmax=1900.0)
+    s = c.scheme
+    k = orc.constants(s, c.vel, dtype=np.float32)
+    ext = (c.rng.standard_normal((nExt, c.nx, c.nz)) * interior_mask(c.nx, c.nz)).astype(np.float32)
+    data = [c.rng.standard_normal((len(r), s.nts)).astype(np.float32) for r in c.rec_pos]
+    out = []
+    for a in ({}, dict(stepper="fine")):
+        ctx = Context(s.nz, s.nx, s.nts, s.dts, s.sub, s.dz, s.dx, s.minPad, k["v2"], k["rs"], nExt=nExt, extension=extension, **a)
+        out.append([np.concatenate([x.ravel() for x in ctx.born_ext_forward(ext, _shots(c))]),
+                    ctx.born_ext_adjoint(_shots(c, data)).ravel().copy()])
+        ctx.close()
+    for a, b in zip(*out):
+        assert np.linalg.norm(b) > 0
+        assert rel_l2(a, b) < 3e-5
