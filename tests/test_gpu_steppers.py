@@ -158,3 +158,34 @@ def test_extended_blocks(nExt, nzi, nxi, nts, extension):
     for a, b in zip(*out):
         assert np.linalg.norm(b) > 0
         assert rel_l2(a, b) < 3e-5
+
+
+def test_staged_models():
+    """Models of 16 MiB and more in pageable memory (packed through pinned buffers) and in pinned memory (copied
+    directly): the same bits, zeros outside the interior, the caller's array added to."""
+    import orc
+    import torch
+    from acoustic_isotropic_operators_b200.batch import Context
+    c = make_case(seed=8, nzi=301, nxi=403, nts=6, sub=4, minPad=6, nshots=1, vmin=1500.0, vmax=1900.0)
+    s = c.scheme
+    k = orc.constants(s, c.vel, dtype=np.float32)
+    ctx = Context(s.nz, s.nx, s.nts, s.dts, s.sub, s.dz, s.dx, s.minPad, k["v2"], k["rs"], nExt=37)
+    mask = interior_mask(c.nx, c.nz)
+    ext = (c.rng.standard_normal((37, c.nx, c.nz)) * mask).astype(np.float32)
+    start = c.rng.standard_normal(ext.shape).astype(np.float32)
+    data = [c.rng.standard_normal((len(r), s.nts)).astype(np.float32) for r in c.rec_pos]
+    out = []
+    for pin in (False, True):
+        own = (lambda a: torch.from_numpy(a).pin_memory().numpy()) if pin else np.copy
+        res = [np.concatenate([x.ravel() for x in ctx.born_ext_forward(own(ext), _shots(c))])]
+        for add in (False, True):
+            m = own(start)
+            ctx.born_ext_adjoint(_shots(c, data), model=m, add=add)
+            res.append(m.copy())
+        out.append(res)
+    ctx.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    edge = np.broadcast_to(mask == 0, ext.shape)
+    assert not out[0][1][edge].any() and np.linalg.norm(out[0][1]) > 0
+    np.testing.assert_array_equal(out[0][2][edge], start[edge])
