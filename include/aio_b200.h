@@ -72,7 +72,8 @@ typedef struct {
     long long memBudgetBytes; /* cap on device memory for shot buffers; 0 = 93% of free */
     int stepper;         /* AIO_STEPPER_*: how Born / nonlinear passes advance time */
     int chunkColumns;    /* blocked stepper x-chunk width: 0 = autotuned (measured once per wave size),
-                            > 0 = fixed width (strips of at most 128 rows) */
+                            > 0 = fixed width (strips of at most 128 rows; narrower where a tile's
+                            devices would not fit) */
     int freeSurface;     /* 1: free surface at the top interior row (reference par freeSurface;
                             the *FsGpu drivers); both steppers */
     int extension;       /* AIO_EXT_*: extension axis of the extended Born / tomo / WEMVA operators
@@ -85,7 +86,7 @@ typedef struct {
 #define AIO_STEPPER_AUTO 0      /* four fine steps per launch where available (sub == 4; nonlinear and Born
                                    operators: sub >= 4), else per fine step */
 #define AIO_STEPPER_FINE 1      /* one fused launch per fine step (the reference's schedule) */
-#define AIO_STEPPER_BLOCKED 2   /* one launch per coarse interval, 2-D register tiles (requires sub == 4) */
+#define AIO_STEPPER_BLOCKED 2   /* one launch per coarse interval (requires sub == 4) */
 
 typedef struct {
     const int* sourcesPositionReg;   /* host array, nSourcesReg */
