@@ -17,6 +17,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "aio_b200.h"
@@ -1526,7 +1527,7 @@ struct Context {
             if (rec == 1) collect(shots[s].receiversPositionReg, shots[s].nReceiversReg, 0, cRec, "receiver");
             if (rec == 2) collect(shots[s].sourcesPositionReg, shots[s].nSourcesReg, 0, cRec, "source");
             for (size_t c = 0; c < nCTA; c++) {
-                auto byKey = [](const KMEnt& A, const KMEnt& B) { return A.key < B.key || (A.key == B.key && A.slot < B.slot); };
+                auto byKey = [](const KMEnt& A, const KMEnt& B) { return std::tie(A.key, A.slot, A.dev) < std::tie(B.key, B.slot, B.dev); };
                 std::sort(cInj[c].begin(), cInj[c].end(), byKey);
                 std::sort(cRec[c].begin(), cRec[c].end(), byKey);
                 int slots = 0;

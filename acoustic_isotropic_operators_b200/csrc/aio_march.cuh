@@ -252,6 +252,18 @@ __device__ __forceinline__ float km_injected(const KMArgs& a, const TBShot& sh, 
     // recursion integrates twice)
     return __fmaf_rn(tr[it], a.h[it2 + 1], __fmul_rn(tr[it + 1], a.h[g.H + it2 + 1]));
 }
+// Value of the point of entry e (of the n from `first` on) at level l into its injection slot. Devices of one point
+// are next to one another in list order, and the first one's thread adds them up in that order: the same sum
+// in every CTA that holds the point, and in every run.
+template <bool ADJ>
+__device__ __forceinline__ void km_slot_value(const KMArgs& a, const TBShot& sh, int first, int n, int e, int l, float4* sV) {
+    const KMEnt* ent = sh.ent + first;
+    const int slot = ent[e].slot;
+    if (e > 0 && ent[e - 1].slot == slot) return;
+    float v = km_injected<ADJ>(a, sh, ent[e].dev, l);
+    for (int k = e + 1; k < n && ent[k].slot == slot; k++) v += km_injected<ADJ>(a, sh, ent[k].dev, l);
+    reinterpret_cast<float*>(sV + (slot >> 2) * KT_T + l - 1)[slot & 3] = v;
+}
 // adds injected values to a quad before its last damping (adjoint recursion: times v^2, product and sum
 // rounded separately but in the nonlinear adjoint)
 template <int MODE>
@@ -777,11 +789,7 @@ __global__ void __launch_bounds__(KM_MAXT, 1) k_march(const KMArgs a) {
     kt_grid_wait();
     if (a.relEarly) kt_grid_release();
     if (!tb_scatlike(MODE)) {
-        for (int k = tid; k < nInj * T; k += nthr) {
-            const int e = k / T, l = k - e * T + 1;
-            const KMEnt en = sh.ent[se.x + e];
-            atomicAdd(reinterpret_cast<float*>(sV + (en.slot >> 2) * T + l - 1) + (en.slot & 3), km_injected<kt_adj(MODE)>(a, sh, en.dev, l));
-        }
+        for (int k = tid; k < nInj * T; k += nthr) km_slot_value<kt_adj(MODE)>(a, sh, se.x, nInj, k / T, k % T + 1, sV);
     }
     const bool zIn = act && zq < g.nzi;
     const bool zOut = zIn && zq >= z0 && zq < z0 + a.HZ;
@@ -911,7 +919,7 @@ __global__ void __launch_bounds__(KB_MAXT, 1) k_block(const KMArgs a) {
     for (int k = tid; k < nInj * T; k += nthr) {
         const int e = k / T, l = k - e * T + 1;
         const KMEnt en = sh.ent[se.x + e];
-        atomicAdd(reinterpret_cast<float*>(sV + (en.slot >> 2) * T + l - 1) + (en.slot & 3), km_injected<UADJ>(a, sh, en.dev, l));
+        km_slot_value<UADJ>(a, sh, se.x, nInj, e, l, sV);
         if (l == 1) slotAt[(en.key >> 16) * CA + (en.key & 0xffff)] = (short)(en.slot >> 2);
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");

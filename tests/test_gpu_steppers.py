@@ -189,3 +189,33 @@ def test_staged_models():
     edge = np.broadcast_to(mask == 0, ext.shape)
     assert not out[0][1][edge].any() and np.linalg.norm(out[0][1]) > 0
     np.testing.assert_array_equal(out[0][2][edge], start[edge])
+
+
+@pytest.mark.parametrize("sub", [4, 6])
+@pytest.mark.parametrize("chunk", [0, 17])
+def test_devices_of_one_point_add_up_in_list_order(chunk, sub):
+    """Devices of one point inject their sum in list order, as the per-fine-step stepper does. Here each sum
+    is of B, v and -B in turn with |v| < |B| 2^-25: exactly zero in that order (B + v = B) and v at least
+    in another one."""
+    import orc
+    from acoustic_isotropic_operators_b200.batch import Context, Shot
+    c = make_case(seed=12, nzi=90, nxi=70, nts=10, sub=sub, minPad=6, nshots=1, vmin=1500.0, vmax=1900.0)
+    s = c.scheme
+    k = orc.constants(s, c.vel, dtype=np.float32)
+    # points around chunk edges and strips, their devices interleaved in the list
+    points = np.array([(5 + ix) * s.nz + 5 + iz for ix in (2, 16, 17, 18, 40, 69) for iz in (0, 3, 45, 89)], np.int32)
+    pos = np.tile(points, 12)
+    rng = np.random.default_rng(5)
+    def traces(n):  # noqa: E306
+        v = rng.standard_normal((4, len(points), n)).astype(np.float32)
+        return np.concatenate([x for t in v for x in (t * np.float32(2.0 ** 27), t, -t * np.float32(2.0 ** 27))])
+    far = np.array([30 * s.nz + 40], np.int32)
+    out = {}
+    for name, a in (("auto", dict(chunk_columns=chunk)), ("fine", dict(stepper="fine"))):
+        ctx = Context(s.nz, s.nx, s.nts, s.dts, s.sub, s.dz, s.dx, s.minPad, k["v2"], k["rs"], **a)
+        rng = np.random.default_rng(5)
+        out[name] = [ctx.nonlinear_forward([Shot(pos, points, traces(s.ntw))])[0],
+                     ctx.nonlinear_adjoint([Shot(far, pos, None, traces(s.nts))])[0]]
+        ctx.close()
+    for x in out["fine"] + out["auto"]:
+        assert not x.any()
