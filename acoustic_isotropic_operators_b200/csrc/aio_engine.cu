@@ -173,7 +173,7 @@ struct Context {
     cudaStream_t st = nullptr;
     DevMem v2, rs, taper;
     float* v2p() const { return v2.as<float>() + (long long)KM_GUARD * g.ip; }  // zero columns around v^2
-    std::vector<float> hv2;  // host copy of v^2 dtw^2, padded grid
+    std::vector<float> hv2;  // host copy of v^2 dtw^2, padded grid; empty: zero everywhere
     // per-wave buffers
     DevMem pbuf, ringb, ssb, wf1, wf2, wf3, img, lists, desc, sig, dat, aux, model, ext, outv;
     std::vector<ShotDesc> hdesc;
@@ -255,6 +255,7 @@ struct Context {
         AIO_CK(cudaSetDevice(dev));
         AIO_CK(cudaMemsetAsync(v2.p, 0, v2.bytes, st));
         AIO_CK(cudaMemsetAsync(rs.p, 0, g.isz * 4, st));
+        hv2.clear();
         if (vel2Dtw2) {
             to_interior(v2p(), vel2Dtw2, 1, AIO_MEM_HOST);
             hv2.assign(vel2Dtw2, vel2Dtw2 + (size_t)g.nz * g.nx);

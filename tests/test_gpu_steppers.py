@@ -219,3 +219,23 @@ def test_devices_of_one_point_add_up_in_list_order(chunk, sub):
         ctx.close()
     for x in out["fine"] + out["auto"]:
         assert not x.any()
+
+
+def test_adjoint_without_velocity():
+    """Where v^2 is zero at a source the nonlinear adjoint keeps the per-fine-step stepper (same bits), also
+    when the velocity was taken away after the context was made."""
+    from acoustic_isotropic_operators_b200 import _capi as A
+    from acoustic_isotropic_operators_b200.batch import Shot
+    c, auto, fine = _pair(40, 50, 4, 0, 2)
+    data = [c.rng.standard_normal((len(r), c.scheme.nts)).astype(np.float32) for r in c.rec_pos]
+    shots = lambda: [Shot(s, np.concatenate([r, s]), None, np.concatenate([d, d[:len(s)]]))  # noqa: E731
+                     for s, r, d in zip(c.src_pos, c.rec_pos, data)]
+    moving = auto.nonlinear_adjoint(shots())
+    for ctx in (auto, fine):
+        A.check(A.lib().aio_context_set_velocity(ctx._h, None, None))
+    for a, b in zip(auto.nonlinear_adjoint(shots()), fine.nonlinear_adjoint(shots())):
+        assert np.isfinite(a).all() and b.any()
+        np.testing.assert_array_equal(a, b)
+    auto.close()
+    fine.close()
+    assert all(x.any() for x in moving)
