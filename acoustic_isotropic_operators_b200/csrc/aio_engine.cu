@@ -478,7 +478,9 @@ struct Context {
     }
     // Waves of (nearly) equal size: ceil(nShots / cap) waves rather than full waves and a
     // small remainder, whose launches would use the GPU poorly.
+    // (a shot is a grid's z index, four of them in k_img_offset_fwd_block: at most 65535)
     static int balanced_wave(long long cap, int nShots) {
+        cap = std::min(cap, 65535LL / 4);
         if (nShots <= cap) return nShots;
         const long long waves = (nShots + cap - 1) / cap;
         return (int)((nShots + waves - 1) / waves);

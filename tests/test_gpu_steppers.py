@@ -239,3 +239,19 @@ def test_adjoint_without_velocity():
     auto.close()
     fine.close()
     assert all(x.any() for x in moving)
+
+
+def test_more_shots_than_a_grid_holds():
+    """More shots than one launch can index (65535) run in waves."""
+    from acoustic_isotropic_operators_b200.batch import Shot
+    c, auto, fine = _pair(11, 13, 4, 0, 3)
+    data = [c.rng.standard_normal((len(r), c.scheme.nts)).astype(np.float32) for r in c.rec_pos]
+    want = fine.nonlinear_adjoint(_shots(c, data))
+    n = 65538
+    got = auto.nonlinear_adjoint([Shot(c.src_pos[i % 3], c.rec_pos[i % 3], None, data[i % 3]) for i in range(n)])
+    for i in range(3):
+        same = np.stack(got[i::3])
+        np.testing.assert_array_equal(same, np.broadcast_to(same[0], same.shape))
+        assert rel_l2(same[0], want[i]) < 2e-5 and want[i].any()
+    auto.close()
+    fine.close()
