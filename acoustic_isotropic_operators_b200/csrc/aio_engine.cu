@@ -494,12 +494,18 @@ struct Context {
             maxSrc = std::max(maxSrc, shots[s].nSourcesReg);
             maxRec = std::max(maxRec, shots[s].nReceiversReg);
         }
+        const size_t wfBytes = (size_t)nb * g.nts * g.isz * 4;
+        if (n.nWavefields + n.nImg > 0)
+            hold_only({{&wf1, n.nWavefields >= 1 ? wfBytes : 0}, {&wf2, n.nWavefields >= 2 ? wfBytes : 0},
+                       {&wf3, n.nWavefields >= 3 ? wfBytes : 0}, {&ssb, n.ss ? (size_t)nb * 2 * g.isz * 4 : 0},
+                       {&img, (size_t)nb * n.nImg * g.isz * (P.imageFp64 ? 8 : 4)}},
+                      {&tbW, &tbState, &tbPart, &tbImg});
         pbuf.ensure((size_t)nb * 2 * g.hsz * 4);
         ringb.ensure((size_t)nb * 2 * g.isz * 4);
         if (n.ss) ssb.ensure((size_t)nb * 2 * g.isz * 4);
-        if (n.nWavefields >= 1) wf1.ensure((size_t)nb * g.nts * g.isz * 4);
-        if (n.nWavefields >= 2) wf2.ensure((size_t)nb * g.nts * g.isz * 4);
-        if (n.nWavefields >= 3) wf3.ensure((size_t)nb * g.nts * g.isz * 4);
+        if (n.nWavefields >= 1) wf1.ensure(wfBytes);
+        if (n.nWavefields >= 2) wf2.ensure(wfBytes);
+        if (n.nWavefields >= 3) wf3.ensure(wfBytes);
         if (n.nImg) img.ensure((size_t)nb * n.nImg * g.isz * (P.imageFp64 ? 8 : 4));
         AIO_CK(cudaMemsetAsync(pbuf.p, 0, (size_t)nb * 2 * g.hsz * 4, st));
         AIO_CK(cudaMemsetAsync(ringb.p, 0, (size_t)nb * 2 * g.isz * 4, st));
@@ -1046,6 +1052,17 @@ struct Context {
         for (DevMem* m : call_buffers()) b += (long long)m->bytes;
         return b;
     }
+    // At sub != 4 an operator's call runs on either stepper, and each keeps its fields in buffers of its own:
+    // those of the other one go where the budget does not hold both. mine: what this wave needs.
+    void hold_only(std::initializer_list<std::pair<DevMem*, size_t>> mine, std::initializer_list<DevMem*> other) {
+        long long b = device_bytes(), held = 0;
+        for (const auto& m : mine) b += std::max(0LL, (long long)m.second - (long long)m.first->bytes);
+        for (const DevMem* o : other) held += (long long)o->bytes;
+        if (!tb_any_sub() || held == 0 || b <= budget) return;
+        AIO_CK(cudaStreamSynchronize(st));
+        drop_graphs();
+        for (DevMem* o : other) o->release();
+    }
     // Frees the per-call buffers (and the captured graphs, whose launches hold their addresses).
     void release_buffers() {
         AIO_CK(cudaSetDevice(dev));
@@ -1574,6 +1591,12 @@ struct Context {
         }
     }
 
+    // a Born wave on the interval steppers
+    void tb_hold(int nb, bool needImg) {
+        hold_only({{&tbW, (size_t)nb * g.nts * g.isz * wbytes()}, {&tbState, (size_t)nb * 4 * g.isz * 4},
+                   {&tbPart, (size_t)nb * tb_parts() * g.isz * 4}, {&tbImg, needImg ? (size_t)nb * g.isz * 8 : 0}},
+                  {&wf1, &wf2, &wf3, &ssb, &img});
+    }
     // Per-shot descriptors and array bases of a pass (launch version v reads state and partial-sum
     // set v and writes set 1-v).
     // wSlices: coarse slices per shot in W (the stored wavefield: nts; a secondary-source ring: its length)
@@ -2462,6 +2485,7 @@ struct Context {
         for (int s0 = 0; s0 < nShots;) {
             const int nb = tb_wave_size(nShots - s0, shots + s0, true, false);
             setup_wave(n, nb, shots + s0, mem, false, false);
+            tb_hold(nb, false);
             tb_alloc(nb, false);
             tbW.ensure((size_t)nb * g.nts * g.isz * wbytes());
             tb_src_pass(nb, shots + s0, false);
@@ -2481,6 +2505,7 @@ struct Context {
         for (int s0 = 0; s0 < nShots;) {
             const int nb = tb_wave_size(nShots - s0, shots + s0, true, true);
             setup_wave(n, nb, shots + s0, mem, true, false);
+            tb_hold(nb, true);
             tb_alloc(nb, true);
             tbW.ensure((size_t)nb * g.nts * g.isz * wbytes());
             tb_src_pass(nb, shots + s0, false);

@@ -255,3 +255,26 @@ def test_more_shots_than_a_grid_holds():
         assert rel_l2(same[0], want[i]) < 2e-5 and want[i].any()
     auto.close()
     fine.close()
+
+
+def test_both_steppers_share_the_budget():
+    """At sub != 4 the Born operators and the extended ones keep their fields on different steppers: a context
+    that runs both in turn stays within its budget."""
+    import orc
+    from acoustic_isotropic_operators_b200.batch import Context, Shot
+    c = make_case(seed=3, nzi=61, nxi=50, nts=300, sub=6, minPad=6, nshots=1, vmin=1500.0, vmax=1900.0)
+    s = c.scheme
+    k = orc.constants(s, c.vel, dtype=np.float32)
+    ctx = Context(s.nz, s.nx, s.nts, s.dts, s.sub, s.dz, s.dx, s.minPad, k["v2"], k["rs"], nExt=3)
+    budget = 200 << 20  # (about 30 of the 40 shots, of 3.8 MB of coarse source field each)
+    ctx.set_budget(budget)
+    data = (c.rng.standard_normal((len(c.rec_pos[0]), s.nts)) * 1e-2).astype(np.float32)
+    shots = [Shot(c.src_pos[0], c.rec_pos[0], c.sig[0], data) for _ in range(40)]
+    out = []
+    for _ in range(2):
+        out.append((ctx.born_adjoint(shots), ctx.born_ext_adjoint(shots)))
+        assert ctx.device_bytes <= budget
+    ctx.close()
+    for a, b in zip(*out):
+        assert a.any()
+        np.testing.assert_array_equal(a, b)
