@@ -388,11 +388,16 @@ struct Context {
                                      src + (long long)e * g.isz, (size_t)g.ip * 4, (size_t)g.nzi * 4, g.nxi, kind, st));
     }
     // Models of at least STAGE_MIN bytes in pageable memory go through two pinned buffers, packed by all host
-    // threads while the other one's copy runs: a pageable copy goes at a single host thread's pace. One B200,
-    // 16 host cores: tomo adjoint of 41 slices of 912 x 3104 points 107.8 -> 77.7 ms. Smaller ones gain less
-    // than the buffers' set-up costs a first call. Pinned (or managed) memory is copied directly, at the
-    // link's pace.
-    static constexpr long long STAGE_BYTES = 8 << 20, STAGE_MIN = 16 << 20;
+    // threads while the other one's copy runs: a pageable copy goes at a single host thread's pace. Pinned (or
+    // managed) memory is copied directly, at the link's pace. Page-locking the buffers takes 14 ms and at times 100,
+    // and staging gains 0.06 (in) to 0.3 ms (out) a MB: a context's models are copied directly up to
+    // STAGE_AFTER bytes in all, so that a first call on a new context pays for them only where it is
+    // large. One B200 on a shared host, ms of a new context's first call, then of each later one; staged from the
+    // first byte, and now: extended adjoint, 31 slices of 300 x 500 points: 39 to 235, 4; 13 to 16, 10 (4 from the
+    // sixth on); forward, 21 slices of 512 x 1312: 38 to 53, 22; 29 to 53, 22 from the third on; tomo adjoint, 41
+    // slices of 912 x 3104: 94 to 233, 77.5; 97 to 103, 77.5 (one copied directly all along: 30 ms more each).
+    static constexpr long long STAGE_BYTES = 8 << 20, STAGE_MIN = 16 << 20, STAGE_AFTER = 80 << 20;
+    long long stageSeen = 0;  // bytes of such models since the context was made or its buffers freed
     struct PinnedBuf {
         float* p = nullptr;
         cudaEvent_t done = nullptr;
@@ -419,7 +424,9 @@ struct Context {
             cudaGetLastError();
             return false;
         }
-        return at.type == cudaMemoryTypeUnregistered && pinned[0].ensure() && pinned[1].ensure();
+        if (at.type != cudaMemoryTypeUnregistered) return false;
+        stageSeen += (long long)nSlices * g.isz * 4;
+        return stageSeen >= STAGE_AFTER && pinned[0].ensure() && pinned[1].ensure();
     }
     // start(buffer, c0, c1, done) for the slices' columns (slice * nxi + x), a buffer at a time; finish(buffer,
     // c0, c1) once its copy is done, after the next one has been started
@@ -1070,6 +1077,7 @@ struct Context {
         drop_graphs();
         for (DevMem* m : call_buffers()) m->release();
         for (PinnedBuf& b : pinned) b.release();
+        stageSeen = 0;
     }
     // Stepper kernels: marching (k_march), a tile per CTA (k_block), sliding blocks (k_slide, dense-source
     // modes at sub = 4). A plan: strips of HZ (multiple of 4) output rows, NQ row quads with their halo,
