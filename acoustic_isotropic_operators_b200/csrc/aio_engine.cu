@@ -1107,10 +1107,11 @@ struct Context {
     TBPlan tb_plan_c(int nb, int cls) const {
         auto it = tbTuned.find(8 * nb + cls);
         if (it != tbTuned.end()) return it->second;
-        // forced chunk width: strips of at most 128 rows
-        if (P.chunkColumns > 0)
-            return tb_make_plan((g.nzi + 127) / 128, std::max(1, (g.nxi + P.chunkColumns / 2) / P.chunkColumns));
-        return tb_candidates(nb, cls, TBEntries{}, 1).front();
+        return P.chunkColumns > 0 ? tb_forced_plan() : tb_candidates(nb, cls, TBEntries{}, 1).front();
+    }
+    // forced chunk width: strips of at most 128 rows
+    TBPlan tb_forced_plan() const {
+        return tb_make_plan((g.nzi + 127) / 128, std::max(1, (g.nxi + P.chunkColumns / 2) / P.chunkColumns));
     }
 
     TBPlan tb_make_plan(int nStrips, int nChunks, int kind = TB_MARCH) const {
@@ -1270,9 +1271,49 @@ struct Context {
         return out;
     }
 
-    std::map<int, TBPlan> tbTuned;
+    std::map<int, TBPlan> tbTuned;  // plan of the class's next pass, by 8 * shots + class (tb_tune)
     TBPlan tbLast;  // plan of the most recent blocked launch
 
+    // Timed plans, by 8 * shots + class and the devices that they were timed for: TB_ANY where every candidate held
+    // them; else, so that a call of few devices is not left with what a call of many had to choose from,
+    // their number, or (none but the smallest tiles held them) their density, within a factor of two.
+    static constexpr int TB_ANY = 0;
+    std::map<std::pair<int, int>, TBPlan> tbTimed;
+    static int tb_octave(int n) {
+        int b = 0;
+        for (; n > 0; n >>= 1) b++;
+        return b;
+    }
+    int tb_count_key(int nb, const aio_shot* shots) const {
+        int n = 0;
+        for (int s = 0; s < nb; s++) n = std::max(n, shots[s].nSourcesReg + shots[s].nReceiversReg);
+        return 1 + tb_octave(n);
+    }
+    int tb_density_key(int nb, const aio_shot* shots) const {
+        const TBEntries e = tb_max_entries(tb_make_plan((g.nzi + 127) / 128, (g.nxi + 63) / 64), nb, shots);
+        return 64 + tb_octave(std::max({e.srcIn, e.recIn, e.srcOut, e.recOut}));
+    }
+    // takes a timed plan that holds these shots' devices: this context's or another one's
+    bool tb_take(int nb, int cls, int devices, const aio_shot* shots) {
+        const int k = 8 * nb + cls;
+        auto it = tbTimed.find({k, devices});
+        TBPlan pl;
+        if (it != tbTimed.end()) {
+            pl = it->second;
+            if (!tb_fits(pl, nb, cls, shots)) return false;
+        } else {
+            {
+                std::lock_guard<std::mutex> lk(shared_plans_mu());
+                auto sh = shared_plans().find(shared_plan_key(k, devices));
+                if (sh == shared_plans().end()) return false;
+                pl = sh->second;
+            }
+            if (tb_occupancy(pl, cls, tb_smem(pl, cls, tb_max_entries(pl, nb, shots))) < 1) return false;
+            tbTimed[{k, devices}] = pl;
+        }
+        tbTuned[k] = pl;
+        return true;
+    }
     // Plans measured by any context of the process, shared by the contexts of the same device,
     // interior size, free-surface setting and stored precision: a new context (a request server
     // opens one per grid and velocity model) takes them instead of timing the candidates again.
@@ -1285,21 +1326,8 @@ struct Context {
         static std::mutex mu;
         return mu;
     }
-    std::vector<int> shared_plan_key(int k) const {
-        return {dev, g.nzi, g.nxi, k, P.freeSurface, P.wavefieldPrecision, tb_any_sub() ? 1 : 0};
-    }
-    // The shared plan of waves of nb shots of a class, when there is one that fits these shots.
-    bool tb_take_shared(int nb, int cls, const aio_shot* shots) {
-        TBPlan pl;
-        {
-            std::lock_guard<std::mutex> lk(shared_plans_mu());
-            auto it = shared_plans().find(shared_plan_key(8 * nb + cls));
-            if (it == shared_plans().end()) return false;
-            pl = it->second;
-        }
-        if (tb_occupancy(pl, cls, tb_smem(pl, cls, tb_max_entries(pl, nb, shots))) < 1) return false;
-        tbTuned[8 * nb + cls] = pl;
-        return true;
+    std::vector<int> shared_plan_key(int k, int devices) const {
+        return {dev, g.nzi, g.nxi, k, devices, P.freeSurface, P.wavefieldPrecision, tb_any_sub() ? 1 : 0};
     }
 
     // CTAs (strip range, chunk range) whose region, widened by h points, holds interior point (z, x)
@@ -1389,35 +1417,35 @@ struct Context {
         return tb_steps() && (!tb_any_sub() || tb_holds(nShots, shots, wavefield, image, classes));
     }
 
-    // Measured autotuning of a class's plan for waves of nb shots (chunkColumns == 0): the dozen
-    // candidates of the smallest modelled time are timed on an idempotent launch of interval 0
-    // (the last interval for ADJ): it reads one state set and overwrites the other, the stored slice
-    // 0 and the partial sums; the fastest is kept for the context and shared with the process.
+    // Measured autotuning of a class's plan for waves of nb shots (chunkColumns == 0): the candidates of the
+    // smallest modelled time (up to 8 tile, 12 sliding-block and 16 marching plans) that hold the devices are
+    // timed on launches of the pass's first four steps, which read one state set and write the other,
+    // the stored slice 0 and the partial sums, all set anew before the pass (recordings are added to the traces,
+    // which are zeroed again); the fastest is kept for the context and shared with the process.
     void tb_tune(int nb, const aio_shot* shots, int cls) {
-        auto known = tbTuned.find(8 * nb + cls);
-        if (known != tbTuned.end()) {
-            if (tb_fits(known->second, nb, cls, shots)) return;
-            tbTuned.erase(known);  // (tuned for fewer devices)
-        }
+        const int k = 8 * nb + cls;
         if (P.chunkColumns > 0) {
-            const TBPlan forced = tb_plan_c(nb, cls);
-            if (!tb_fits(forced, nb, cls, shots)) {
-                TBPlan pl;
-                require(tb_dense_plan(nb, cls, shots, forced.nStrips, forced.nChunks, pl), "blocked stepper: too many sparse devices inside one tile");
-                tbTuned[8 * nb + cls] = pl;
-            }
+            TBPlan pl = tb_forced_plan();
+            require(tb_fits(pl, nb, cls, shots) || tb_dense_plan(nb, cls, shots, pl.nStrips, pl.nChunks, pl),
+                    "blocked stepper: too many sparse devices inside one tile");
+            tbTuned[k] = pl;
             return;
         }
-        if (tb_take_shared(nb, cls, shots)) return;
-        // device counts enter the candidates' shared memory: those of a mid-sized tile, then checked
-        // exactly per candidate
+        const int count = tb_count_key(nb, shots);
+        if (tb_take(nb, cls, TB_ANY, shots) || tb_take(nb, cls, count, shots)) return;
+        const int density = tb_density_key(nb, shots);
+        if (tb_take(nb, cls, density, shots)) return;
         std::vector<TBPlan> cand;
-        for (const TBPlan& pl : tb_tile_candidates(nb, cls, 8))
-            if (tb_occupancy(pl, cls, tb_smem(pl, cls, tb_max_entries(pl, nb, shots))) >= 1) cand.push_back(pl);
-        for (const TBPlan& pl : tb_slide_candidates(nb, cls))
-            if (tb_occupancy(pl, cls, tb_smem(pl, cls, tb_max_entries(pl, nb, shots))) >= 1) cand.push_back(pl);
-        for (const TBPlan& pl : tb_candidates(nb, cls, TBEntries{}, 16))
-            if (tb_occupancy(pl, cls, tb_smem(pl, cls, tb_max_entries(pl, nb, shots))) >= 1) cand.push_back(pl);
+        bool all = true;  // every candidate holds the devices
+        auto add = [&](const std::vector<TBPlan>& plans) {
+            for (const TBPlan& pl : plans) {
+                if (tb_occupancy(pl, cls, tb_smem(pl, cls, tb_max_entries(pl, nb, shots))) >= 1) cand.push_back(pl);
+                else if (tb_occupancy(pl, cls, tb_smem(pl, cls, TBEntries{})) >= 1) all = false;
+            }
+        };
+        add(tb_tile_candidates(nb, cls, 8));
+        add(tb_slide_candidates(nb, cls));
+        add(tb_candidates(nb, cls, TBEntries{}, 16));
         const bool dense = cand.empty();
         if (dense) {
             cand.resize(1);
@@ -1510,10 +1538,10 @@ struct Context {
         launches = saveLaunches;
         kernels = saveKernels;
         profEvery = saveProf;
-        tbTuned[8 * nb + cls] = best;
-        if (dense) return;  // (not for contexts with fewer devices)
+        const int devices = dense ? density : (all ? TB_ANY : count);
+        tbTuned[k] = tbTimed[{k, devices}] = best;
         std::lock_guard<std::mutex> lk(shared_plans_mu());
-        shared_plans().emplace(shared_plan_key(8 * nb + cls), best);
+        shared_plans()[shared_plan_key(k, devices)] = best;
     }
     // Per-CTA sparse lists of every shot of a wave. inj: 0 none, 1 sources, 2 receivers
     // (over the CTA's recomputed halo region); rec: 0 none, 1 receivers, 2 sources recorded (output region). Entries are

@@ -280,3 +280,34 @@ def test_both_steppers_share_the_budget():
     for a, b in zip(*out):
         assert a.any()
         np.testing.assert_array_equal(a, b)
+
+
+def test_few_devices_after_many(monkeypatch, capfd):
+    """A call of few devices is not left with the plan that a call of many had to take, in the same context
+    or in another one of the process; neither is timed twice. (The grids are this test's own.)"""
+    import orc
+    from acoustic_isotropic_operators_b200.batch import Context, Shot
+    monkeypatch.setenv("AIO_AUTOTUNE_LOG", "1")
+    c = make_case(seed=4, nzi=214, nxi=204, nts=8, sub=4, minPad=6, nshots=1, vmin=1500.0, vmax=1900.0)
+    s = c.scheme
+    k = orc.constants(s, c.vel, dtype=np.float32)
+    points = np.array([[ix * s.nz + iz for iz in range(5, s.nz - 5)] for ix in range(5, s.nx - 5)], np.int32)
+    # held by every, by some and by none of the timed tiles
+    few, some, many = points[70, 60:63], points[60:160, 60:130].ravel(), points.ravel()
+    ctx = [Context(s.nz, s.nx, s.nts, s.dts, s.sub, s.dz, s.dx, s.minPad, k["v2"], k["rs"]) for _ in range(3)]
+
+    def plan(i, pos):
+        capfd.readouterr()
+        data = np.zeros((len(pos), s.nts), np.float32)
+        ctx[i].nonlinear_adjoint([Shot(c.src_pos[0], pos, None, data) for _ in range(6)])
+        return ctx[i].blocked_plan(0), capfd.readouterr().err.count("aio autotune")
+
+    first = plan(0, many), plan(0, some), plan(0, few)
+    assert first[0][1] == 0 and 0 < first[1][1] < first[2][1]
+    plans = [p for p, _ in first]
+    for i, pos, want in ((0, some, plans[1:]), (0, few, plans[2:]), (0, many, plans[:1]),
+                         (1, many, plans[:1]), (1, few, plans[2:]), (2, some, plans[1:]), (2, few, plans[2:])):
+        got, timed = plan(i, pos)
+        assert got in want and timed == 0
+    for x in ctx:
+        x.close()
