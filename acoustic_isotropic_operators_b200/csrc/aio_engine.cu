@@ -232,6 +232,10 @@ struct Context {
         // every CTA has passed its dependency wait; 2: once every CTA has begun its last iteration
         const char* pEnv = std::getenv("AIO_PDL");
         if (pEnv && pEnv[0] >= '0' && pEnv[0] <= '2') pdlMode = pEnv[0] - '0';
+        // AIO_PLANS=march, tile or slide: only plans of that stepper kernel, where a class has any (tests compare them)
+        const char* kEnv = std::getenv("AIO_PLANS");
+        const std::string only = kEnv ? kEnv : "";
+        onlyKind = only == "march" ? TB_MARCH : (only == "tile" ? TB_TILE : (only == "slide" ? TB_SLIDE : -1));
         live_contexts()[dev & 63]++;
         counted = true;
     }
@@ -1083,6 +1087,7 @@ struct Context {
     // modes at sub = 4). A plan: strips of HZ (multiple of 4) output rows, NQ row quads with their halo,
     // x-chunks of LX columns.
     enum TBKind { TB_MARCH = 0, TB_TILE = 1, TB_SLIDE = 2 };
+    int onlyKind = -1;  // of timed plans; -1: all
     struct TBPlan {
         int T = KT_T, HZ = 0, nStrips = 0, LX = 0, nChunks = 0, NQ = 0;
         int kind = TB_MARCH;  // stepper kernel
@@ -1327,7 +1332,7 @@ struct Context {
         return mu;
     }
     std::vector<int> shared_plan_key(int k, int devices) const {
-        return {dev, g.nzi, g.nxi, k, devices, P.freeSurface, P.wavefieldPrecision, tb_any_sub() ? 1 : 0};
+        return {dev, g.nzi, g.nxi, k, devices, P.freeSurface, P.wavefieldPrecision, tb_any_sub() ? 1 : 0, onlyKind};
     }
 
     // CTAs (strip range, chunk range) whose region, widened by h points, holds interior point (z, x)
@@ -1443,9 +1448,9 @@ struct Context {
                 else if (tb_occupancy(pl, cls, tb_smem(pl, cls, TBEntries{})) >= 1) all = false;
             }
         };
-        add(tb_tile_candidates(nb, cls, 8));
-        add(tb_slide_candidates(nb, cls));
-        add(tb_candidates(nb, cls, TBEntries{}, 16));
+        if (onlyKind < 0 || onlyKind == TB_TILE) add(tb_tile_candidates(nb, cls, 8));
+        if (onlyKind < 0 || onlyKind == TB_SLIDE) add(tb_slide_candidates(nb, cls));
+        if (onlyKind < 0 || onlyKind == TB_MARCH || cand.empty()) add(tb_candidates(nb, cls, TBEntries{}, 16));
         const bool dense = cand.empty();
         if (dense) {
             cand.resize(1);

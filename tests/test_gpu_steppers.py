@@ -52,7 +52,7 @@ def test_against_fine_steps(nzi, nxi, shots, sub, fs):
 
 @pytest.mark.parametrize("nzi,nxi,shots", SIZES)
 def test_dense_source_passes(nzi, nxi, shots):
-    """Tomo and WEMVA (dense sources, stored samples), timed plans."""
+    """Tomo (dense sources, stored samples), timed plans."""
     c, blocked, fine = _pair(nzi, nxi, 4, 0, shots, nExt=3)
     ext = (c.rng.standard_normal((3, c.nx, c.nz)) * interior_mask(c.nx, c.nz)).astype(np.float32)
     data = [c.rng.standard_normal((len(r), c.scheme.nts)).astype(np.float32) for r in c.rec_pos]
@@ -311,3 +311,46 @@ def test_few_devices_after_many(monkeypatch, capfd):
         assert got in want and timed == 0
     for x in ctx:
         x.close()
+
+
+# as SIZES, wide enough for several plans of every kind (a tile's chunks are a multiple of four columns, of 8 at least)
+KIND_SIZES = [(21, 48, 1), (33, 40, 3), (128, 64, 2), (129, 61, 1), (301, 45, 2), (67, 530, 1), (530, 32, 1)]
+
+
+@pytest.mark.parametrize("nzi,nxi,shots,fs,wavefield",
+                         [(*s, fs, "fp32") for s in KIND_SIZES for fs in (0, 1)] +
+                         [(*s, fs, w) for s in KIND_SIZES[2:5] for fs in (0, 1) for w in ("bf16", "fp16")])
+def test_stepper_kernels_agree(nzi, nxi, shots, fs, wavefield, monkeypatch, capfd):
+    """The marching, tile and sliding-block kernels give the same bits at sub = 4 in every operator, so that the
+    timed choice between them changes no result. (The sliding blocks run the dense-source passes only.)"""
+    import orc
+    from acoustic_isotropic_operators_b200.batch import Context, Shot
+    monkeypatch.setenv("AIO_AUTOTUNE_LOG", "1")
+    c = make_case(seed=nzi + 7, nzi=nzi, nxi=nxi, nts=14, sub=4, minPad=6, nshots=shots, vmin=1500.0, vmax=1900.0)
+    s = c.scheme
+    k = orc.constants(s, c.vel, dtype=np.float32)
+    ext = (c.rng.standard_normal((3, c.nx, c.nz)) * interior_mask(c.nx, c.nz)).astype(np.float32)
+    data = [c.rng.standard_normal((len(r), s.nts)).astype(np.float32) for r in c.rec_pos]
+    wemva = lambda: [Shot(c.src_pos[i], c.rec_pos[i], c.sig[i], None, data[i]) for i in range(shots)]  # noqa: E731
+    out = {}
+    for kind in ("march", "tile", "slide"):
+        monkeypatch.setenv("AIO_PLANS", kind)
+        capfd.readouterr()
+        ctx = Context(s.nz, s.nx, s.nts, s.dts, s.sub, s.dz, s.dx, s.minPad, k["v2"], k["rs"], nExt=3, free_surface=fs,
+                      wavefield=wavefield)
+        flat = lambda x: np.concatenate([a.ravel() for a in x])  # noqa: E731
+        out[kind] = {"nl fwd": flat(ctx.nonlinear_forward(_shots(c))), "nl adj": flat(ctx.nonlinear_adjoint(_shots(c, data))),
+                     "born fwd": flat(ctx.born_forward(ext[1], _shots(c))), "born adj": ctx.born_adjoint(_shots(c, data)),
+                     "ext fwd": flat(ctx.born_ext_forward(ext, _shots(c))), "ext adj": ctx.born_ext_adjoint(_shots(c, data)),
+                     "tomo fwd": flat(ctx.tomo_forward(ext[1], ext, _shots(c))),
+                     "tomo adj": ctx.tomo_adjoint(ext, _shots(c, data)),
+                     "wemva fwd": ctx.wemva_forward(ext[1], wemva()), "wemva adj": ctx.wemva_adjoint(ext, wemva())}
+        ctx.close()
+        log = [x for x in capfd.readouterr().err.splitlines() if x.startswith("aio autotune")]
+        # classes: light 0, heavy 1, receiver 2, nonlinear 3 and 4, dense 5
+        own = [x.split("class ")[1][0] for x in log if (f"({kind})" in x if kind != "march" else "(" not in x)]
+        assert set(own) == (set("15") if kind == "slide" else set("012345"))
+    for kind in ("tile", "slide"):
+        for op, want in out["march"].items():
+            assert want.any(), op
+            np.testing.assert_array_equal(out[kind][op], want, err_msg=f"{kind} {op}")
