@@ -17,7 +17,8 @@ that driver on the same m and d. One JSON line per size is printed (the committe
 assembled from these lines). Gates: nrel <= 1e-6 on every draw (a consistent FP32 adjoint pair
 sits near 1e-8 there; a wrong adjoint term would show at 1e-3 or more), and the median rel of
 this engine within the reach of the FP32 round-off the reference's own drivers show on the same
-draws: at most 5 times their median, or 1e-5.
+draws: at most 5 times their median (measured beside it, or where those drivers are not built the
+median they had on these draws, REF_MEDIAN, for the longest run), or 1e-5.
 """
 import json
 
@@ -101,6 +102,10 @@ def _nl_grid():
     return s, w.vel, [(a.src_pos, a.rec_pos, None)]
 
 
+# Median rel of the reference's FP32 drivers on these very draws (seed 17, one B200), for the size where the bound
+# without them, 1e-5, is below what round-off gives: 7996 fine steps, twice the next longest run's.
+REF_MEDIAN = {"born 512x1312 nts=2000": 4.6e-6}
+
 # (label, operator, problem)
 SIZES = [
     ("born 48x64 nts=40 sub=3", "born", lambda: _small(40, 3)),
@@ -136,5 +141,5 @@ def test_dot_curve(label, op, problem):
                     ref_nrel_max=float(theirs[:, 1].max()))
     print(json.dumps(line))
     assert ours[:, 1].max() <= 1e-6
-    bound = max(5 * line["ref_rel_median"], 1e-5) if ref else 1e-5
+    bound = max(5 * (line["ref_rel_median"] if ref else REF_MEDIAN.get(label, 0.0)), 1e-5)
     assert line["rel_median"] <= bound
