@@ -1354,6 +1354,7 @@ struct Context {
         std::vector<int> n(nCTA), pts;
         TBEntries m;
         auto most = [&](const int* pos, int cnt, int h, int& out) {
+            if (!pos || cnt <= 0) return;  // (no list: no devices, as append_list)
             std::fill(n.begin(), n.end(), 0);
             if (h > 0) {  // injected devices of one point share a slot
                 pts.assign(pos, pos + cnt);
@@ -1372,7 +1373,7 @@ struct Context {
             most(shots[s].sourcesPositionReg, shots[s].nSourcesReg, 0, m.srcOut);
             // warps of level 4 (32 row quads each) that record in some CTA: of the widest strip
             std::vector<unsigned char> has((size_t)pl.nStrips * km_warps(pl.NQ), 0);
-            for (int k2 = 0; k2 < shots[s].nReceiversReg; k2++) {
+            for (int k2 = 0; shots[s].receiversPositionReg && k2 < shots[s].nReceiversReg; k2++) {
                 const int z = shots[s].receiversPositionReg[k2] % g.nz - FAT, st2 = z / pl.HZ;
                 if (z >= 0 && z < g.nzi) has[(size_t)st2 * km_warps(pl.NQ) + (z - strip_begin(pl, st2)) / 128] = 1;
             }
@@ -1566,7 +1567,7 @@ struct Context {
             for (auto& v : cInj) v.clear();
             for (auto& v : cRec) v.clear();
             auto collect = [&](const int* pos, int n, int h, std::vector<std::vector<KMEnt>>& out, const char* what) {
-                for (int k2 = 0; k2 < n; k2++) {
+                for (int k2 = 0; pos && k2 < n; k2++) {
                     const long long p = pos[k2];
                     const int iz = (int)(p % g.nz), ix = (int)(p / g.nz);
                     require(p >= 0 && ix < g.nx && iz >= FAT && iz < g.nz - FAT && ix >= FAT && ix < g.nx - FAT,
@@ -1935,7 +1936,7 @@ struct Context {
     // v^2 is positive at every source position (U / v2 is the field there)
     bool sources_move(int nShots, const aio_shot* shots) const {
         for (int s = 0; s < nShots; s++)
-            for (int k2 = 0; k2 < shots[s].nSourcesReg; k2++) {
+            for (int k2 = 0; shots[s].sourcesPositionReg && k2 < shots[s].nSourcesReg; k2++) {
                 const long long p = shots[s].sourcesPositionReg[k2];
                 if (p < 0 || p >= (long long)hv2.size() || !(hv2[p] > 0.f)) return false;
             }

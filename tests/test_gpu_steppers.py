@@ -243,6 +243,25 @@ def test_adjoint_without_velocity():
     assert all(x.any() for x in moving)
 
 
+@pytest.mark.parametrize("sub", [4, 6])
+def test_counts_without_positions(sub):
+    """A device count without positions is no device, on either stepper."""
+    from acoustic_isotropic_operators_b200 import _capi as A
+    c, auto, fine = _pair(40, 50, sub, 0, 1)
+    s = c.scheme
+    pos, data = c.rec_pos[0], c.rng.standard_normal((len(c.rec_pos[0]), s.nts)).astype(np.float32)
+    sig, out = np.ones((2, s.ntw), np.float32), []
+    for ctx in (auto, fine):
+        res = np.full((len(pos), s.nts), 7.0, np.float32), np.full((2, s.ntw), 7.0, np.float32)
+        A.check(A.lib().aio_nonlinear_forward(ctx._h, 1, (A.AioShot * 1)(A.AioShot(
+            None, 2, A.iptr(pos), len(pos), A.fptr(sig), A.fptr(res[0]), None, None)), A.AIO_MEM_HOST))
+        A.check(A.lib().aio_nonlinear_adjoint(ctx._h, 1, (A.AioShot * 1)(A.AioShot(
+            None, 2, A.iptr(pos), len(pos), None, A.fptr(data), None, A.fptr(res[1]))), A.AIO_MEM_HOST))
+        out += res
+        ctx.close()
+    assert not any(x.any() for x in out)
+
+
 def test_more_shots_than_a_grid_holds():
     """More shots than one launch can index (65535) run in waves."""
     from acoustic_isotropic_operators_b200.batch import Shot
