@@ -1595,7 +1595,10 @@ struct Context {
                 int slots = 0;
                 for (size_t e = 0; e < cInj[c].size(); e++) {
                     if (e == 0 || cInj[c][e].key != cInj[c][e - 1].key) slots++;
-                    cInj[c][e].slot |= (slots - 1) << 2;
+                    const int row = cInj[c][e].slot;
+                    const bool first = e == 0 || cInj[c][e].key != cInj[c][e - 1].key || row != (cInj[c][e - 1].slot & 3);
+                    if (!first) cInj[c][e - 1].slot |= KM_MORE;
+                    cInj[c][e].slot = (slots - 1) << KM_SLOT | (first ? KM_FIRST : 0) | row;
                 }
                 m.maxInj = std::max(m.maxInj, slots);
                 m.maxRec = std::max(m.maxRec, (int)cRec[c].size());

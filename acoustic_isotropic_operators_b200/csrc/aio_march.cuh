@@ -252,17 +252,21 @@ __device__ __forceinline__ float km_injected(const KMArgs& a, const TBShot& sh, 
     // recursion integrates twice)
     return __fmaf_rn(tr[it], a.h[it2 + 1], __fmul_rn(tr[it + 1], a.h[g.H + it2 + 1]));
 }
-// Value of the point of entry e (of the n from `first` on) at level l into its injection slot. Devices of one point
-// are next to one another in list order, and the first one's thread adds them up in that order: the same sum
-// in every CTA that holds the point, and in every run.
+// Value of the point of entry e at level l into its injection slot. Devices of one point are next to one
+// another in list order, and the first one's thread adds them up in that order: the same sum in every CTA that
+// holds the point, and in every run.
 template <bool ADJ>
-__device__ __forceinline__ void km_slot_value(const KMArgs& a, const TBShot& sh, int first, int n, int e, int l, float4* sV) {
-    const KMEnt* ent = sh.ent + first;
-    const int slot = ent[e].slot;
-    if (e > 0 && ent[e - 1].slot == slot) return;
-    float v = km_injected<ADJ>(a, sh, ent[e].dev, l);
-    for (int k = e + 1; k < n && ent[k].slot == slot; k++) v += km_injected<ADJ>(a, sh, ent[k].dev, l);
-    reinterpret_cast<float*>(sV + (slot >> 2) * KT_T + l - 1)[slot & 3] = v;
+__device__ __forceinline__ void km_slot_value(const KMArgs& a, const TBShot& sh, const KMEnt* ent, int e, const KMEnt& en, int l,
+                                              float4* sV) {
+    if (!(en.slot & KM_FIRST)) return;
+    float v = km_injected<ADJ>(a, sh, en.dev, l);
+#pragma unroll 1
+    for (int more = en.slot & KM_MORE; more;) {
+        const KMEnt next = ent[++e];
+        v += km_injected<ADJ>(a, sh, next.dev, l);
+        more = next.slot & KM_MORE;
+    }
+    reinterpret_cast<float*>(sV + (en.slot >> KM_SLOT) * KT_T + l - 1)[en.slot & 3] = v;
 }
 // adds injected values to a quad before its last damping (adjoint recursion: times v^2, product and sum
 // rounded separately but in the nonlinear adjoint)
@@ -761,7 +765,7 @@ __global__ void __launch_bounds__(KM_MAXT, 1) k_march(const KMArgs a) {
     }
     const int4 se = sh.entStart[strip * a.nChunks + chunk];
     const int nInj = se.y - se.x, nRec = se.w - se.z;
-    const int nSlots = nInj > 0 ? (sh.ent[se.y - 1].slot >> 2) + 1 : 0;
+    const int nSlots = nInj > 0 ? (sh.ent[se.y - 1].slot >> KM_SLOT) + 1 : 0;
     for (int k = tid; k < NQ; k += nthr) first[k] = nSlots;
     for (int k = tid; k <= km_warps(NQ); k += nthr) firstRec[k] = nRec;
     for (int k = tid; k < nSlots * T; k += nthr) sV[k] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -774,8 +778,8 @@ __global__ void __launch_bounds__(KM_MAXT, 1) k_march(const KMArgs a) {
     __syncthreads();
     for (int e = tid; e < nInj; e += nthr) {
         const KMEnt en = sh.ent[se.x + e];
-        sKey[en.slot >> 2] = en.key;
-        if (e == 0 || (sh.ent[se.x + e - 1].key >> 16) != (en.key >> 16)) first[en.key >> 16] = en.slot >> 2;
+        sKey[en.slot >> KM_SLOT] = en.key;
+        if (e == 0 || (sh.ent[se.x + e - 1].key >> 16) != (en.key >> 16)) first[en.key >> 16] = en.slot >> KM_SLOT;
     }
     for (int e = tid; e < nRec; e += nthr) {
         const KMEnt en = sh.ent[se.z + e];
@@ -785,11 +789,18 @@ __global__ void __launch_bounds__(KM_MAXT, 1) k_march(const KMArgs a) {
         for (int k = e == 0 ? 0 : (sh.ent[se.z + e - 1].key >> 16) + 1; k <= en.key >> 16; k++) firstRec[k] = e;
     }
     if (tid == 0) sKey[nSlots] = -1;
+    KMEnt mine = {};  // the first entry that this thread injects
+    if (!tb_scatlike(MODE) && tid < nInj * T) mine = sh.ent[se.x + tid / T];
     // ---- everything below reads what the previous launch of the stream wrote
     kt_grid_wait();
     if (a.relEarly) kt_grid_release();
     if (!tb_scatlike(MODE)) {
-        for (int k = tid; k < nInj * T; k += nthr) km_slot_value<kt_adj(MODE)>(a, sh, se.x, nInj, k / T, k % T + 1, sV);
+#pragma unroll 1
+        for (int k = tid; k < nInj * T; k += nthr) {
+            const int e = k / T, l = k - e * T + 1;
+            const KMEnt en = k == tid ? mine : sh.ent[se.x + e];
+            km_slot_value<kt_adj(MODE)>(a, sh, sh.ent + se.x, e, en, l, sV);
+        }
     }
     const bool zIn = act && zq < g.nzi;
     const bool zOut = zIn && zq >= z0 && zq < z0 + a.HZ;
@@ -897,7 +908,7 @@ __global__ void __launch_bounds__(KB_MAXT, 1) k_block(const KMArgs a) {
         const int z = zb + k, dd = z < 0 ? -1 : (FS ? g.nzi - 1 - z : min(z, g.nzi - 1 - z));  // free surface: no top taper
         reinterpret_cast<float*>(dzt)[k] = dd < 0 ? 0.f : (dd < g.minPad ? __ldg(a.taper + dd) : 1.f);
     }
-    const int nSlots = nInj > 0 ? (sh.ent[se.y - 1].slot >> 2) + 1 : 0;
+    const int nSlots = nInj > 0 ? (sh.ent[se.y - 1].slot >> KM_SLOT) + 1 : 0;
     for (int k = tid; k < nSlots * T; k += nthr) sV[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
     // ---- everything below reads what the previous launch of the stream wrote
@@ -919,8 +930,8 @@ __global__ void __launch_bounds__(KB_MAXT, 1) k_block(const KMArgs a) {
     for (int k = tid; k < nInj * T; k += nthr) {
         const int e = k / T, l = k - e * T + 1;
         const KMEnt en = sh.ent[se.x + e];
-        km_slot_value<UADJ>(a, sh, se.x, nInj, e, l, sV);
-        if (l == 1) slotAt[(en.key >> 16) * CA + (en.key & 0xffff)] = (short)(en.slot >> 2);
+        km_slot_value<UADJ>(a, sh, sh.ent + se.x, e, en, l, sV);
+        if (l == 1) slotAt[(en.key >> 16) * CA + (en.key & 0xffff)] = (short)(en.slot >> KM_SLOT);
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();

@@ -42,9 +42,11 @@ enum TBWfld { TBW_F32 = 0, TBW_BF16 = 1, TBW_F16 = 2 };
 // slot: their values are added up in shared memory before the march.
 struct KMEnt {
     int key;    // injection: row quad of the CTA << 16 | column - xs; recording: quad / 32 << 16 | column - xs
-    int slot;   // injection slot << 2 | row of the quad; recording: quad % 32 << 2 | row
+    int slot;   // injection slot << KM_SLOT | KM_FIRST and KM_MORE | row of the quad; recording: quad % 32 << 2 | row
     int dev;    // trace index
 };
+
+constexpr int KM_SLOT = 4, KM_MORE = 4, KM_FIRST = 8;  // the first entry of a point; the next one is of the same point
 
 struct TBShot {
     const float* injSig;  // sparse injection traces
