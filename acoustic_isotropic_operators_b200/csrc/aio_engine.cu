@@ -1094,8 +1094,10 @@ struct Context {
     };
 
     bool tb_enabled() const { return P.stepper != AIO_STEPPER_FINE && g.sub == KT_T; }
-    // The nonlinear and Born passes run blocked whenever a launch's four fine steps span at most two
-    // coarse intervals. (Below that, sub = 2 and 3, a launch would finish two samples.) See tb_runs.
+    // The nonlinear and Born passes run blocked from sub = 4 on: a launch's four fine steps then finish at most one
+    // coarse sample, and the source and receiver passes (KMOut::write) store or image one per launch. At sub = 2
+    // and 3 they would finish two. The nonlinear passes store none and could run there as they are; that has
+    // not been built into the dispatch or timed, and they keep the per-fine-step stepper. See tb_runs.
     bool tb_steps() const { return P.stepper != AIO_STEPPER_FINE && g.sub >= KT_T; }
     bool tb_any_sub() const { return g.sub != KT_T; }
     int tb_launches() const { return ((g.nts - 1) * g.sub + KT_T - 1) / KT_T; }
@@ -2101,7 +2103,9 @@ struct Context {
         return P.wavefieldPrecision == AIO_WFLD_BF16 ? TBW_BF16 : (P.wavefieldPrecision == AIO_WFLD_FP16 ? TBW_F16 : TBW_F32);
     }
 
-    // (a limit of earlier kernels' shared memory)
+    // The longest extension that the blocked operators take. (The register window of the lag kernels sets no
+    // such limit; it is that of their first form, which held the window in shared memory, kept because
+    // nothing longer has been run or sized for.)
     void require_lags(int hExt) const { require(hExt <= 92, "extension too long for the blocked lag imaging"); }
     // f(precision, sign) with both as constants
     template <class F>

@@ -11,12 +11,12 @@
 // formed once per column, at level 1, and kept in two rings of 32 columns.
 //
 // The marching stepper (aio_march.cuh) needs fewer instructions and barriers per update, but its dense-source
-// modes hold 24 columns of both source slices for every row: at most 384 rows per SM, so strips that do
+// modes hold 33 columns of both source slices for every row: at most 384 rows per SM, so strips that do
 // not fill its warps (32 row quads) leave them idle, and its 52 columns of filling weigh on narrow chunks.
-// Measured on one B200, this stepper against the best plan of the others: tomo adjoint, 21 shots of
-// 78 x 569 points: 25.4 against 33.5 ms; Born forward, 11 shots of 386 x 267: 32.4 against 36.7 ms;
-// Born forward, 32 shots of 512 x 1312 (SCAT): 0.48 against 0.33 ms per launch. The plan is chosen by timing.
-// Same bits either way.
+// Measured on one B200, whole calls with the dense passes on this stepper, and on the marching one: tomo adjoint,
+// one shot of 912 x 3104 points, nts = 100: 35.7 and 44.2 ms; 21 shots of 78 x 569, nts = 200: 33.3 and 42.9;
+// Born forward, 11 shots of 386 x 267, nts = 400: 26.0 and 31.2; 32 shots of 512 x 1312, nts = 100: 70.5 and
+// 77.7 (0.40 and 0.47 ms per scattering launch). The plan is chosen by timing. Same bits either way.
 #pragma once
 #include "aio_march.cuh"
 

@@ -202,7 +202,9 @@ def run_reference(args):
 
 def kernel_name(args, w):
     if args.stepper != "fine" and w.sub == 4:
-        return "k_march / k_slide (interval steppers, one launch per coarse interval)"
+        return "k_march / k_block / k_slide (interval steppers, one launch per coarse interval)"
+    if args.stepper == "auto" and w.sub > 4:
+        return "k_march / k_block (interval steppers, four fine steps per launch)"
     return "k_step (fused fine-step stepper)"
 
 
@@ -616,9 +618,11 @@ def main():
     tr = os.path.join(ROOT, "profiles", "stepper_traffic.json")
     if os.path.exists(tr):
         try:
-            byp = json.load(open(tr))["bytes_per_point_update"]
+            captured = json.load(open(tr))
+            byp = captured["bytes_per_point_update"]
             key = args.wavefield if args.image == "fp32" else args.wavefield + "_fp64_image"
-            traffic = byp[key] * launch_pts if key in byp else None
+            if captured["kernel"] == kernel_name(args, w) and not args.chunk:  # (timed plans)
+                traffic = byp[key] * launch_pts if key in byp else None
         except Exception:
             traffic = None
 

@@ -34,3 +34,15 @@ def test_reference_arm_line():
     assert line["e2e"]["h2d_bytes_per_step"] == 0 and line["e2e"]["d2h_bytes_per_step"] == 0
     assert line["config"]["workload"].startswith("batched Born forward+adjoint")
     assert "PRODUCT_NOT_LOADED" in out.stdout
+
+
+def test_traffic_is_of_the_timed_kernel():
+    """The captured DRAM bytes that the line prints name the kernel that the default workload runs."""
+    import types
+    sys.path.insert(0, ROOT)
+    import bench
+    captured = json.load(open(os.path.join(ROOT, "profiles", "stepper_traffic.json")))
+    w = types.SimpleNamespace(sub=4)
+    assert captured["kernel"] == bench.kernel_name(types.SimpleNamespace(stepper="auto"), w)
+    assert captured["kernel"] != bench.kernel_name(types.SimpleNamespace(stepper="fine"), w)
+    assert {"fp32", "bf16", "fp16"} <= set(captured["bytes_per_point_update"])
