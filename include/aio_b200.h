@@ -81,7 +81,8 @@ typedef struct {
 } aio_params;
 
 #define AIO_EXT_TIME 0      /* time lags (the *TimeShots* drivers) */
-#define AIO_EXT_OFFSET 1    /* horizontal subsurface offsets (the *OffsetShots* drivers; per-fine-step stepper) */
+#define AIO_EXT_OFFSET 1    /* horizontal subsurface offsets (the *OffsetShots* drivers; tomo and WEMVA per
+                               fine step) */
 
 #define AIO_STEPPER_AUTO 0      /* four fine steps per launch where available (sub == 4; nonlinear and Born
                                    operators: sub >= 4), else per fine step */
